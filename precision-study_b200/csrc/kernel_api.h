@@ -31,8 +31,9 @@ enum Precision : int { PREC_FP64 = 0, PREC_FP32 = 1, PREC_MIXED = 2 };
 #endif
 constexpr int kTileHeights[2] = {PMHD_TY0, 8};
 constexpr int kNumTileHeights = 2;
-// A batched stage launch hands its CTAs runs of this many consecutive tiles.
-constexpr int kBatchRun = 16;
+// A batched stage launch hands its CTAs runs of consecutive tiles, at most
+// this many (a power of two; see batch_run in kernels.cu).
+constexpr int kBatchRunMax = 16;
 
 // One grid of a batch; lives in device memory (64-byte aligned for the TMA
 // descriptors).

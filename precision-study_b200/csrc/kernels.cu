@@ -87,13 +87,29 @@ static int occupancy() {
   return per_sm;
 }
 
+// Tiles per run of a batched launch of `ntiles` tiles on `grid` CTAs: the
+// longest run (fewest re-reads of member descriptors and control slots) whose
+// busiest CTA gets at most 1/16 more tiles than it would with runs of one.
+// Short work lists need short runs: 16 members of 64^2 .. 256^2 (700 tiles on
+// 148 CTAs) as runs of 16 keep 44 CTAs busy; long lists (the 512-member
+// benchmark ensemble, 73,000 tiles) keep runs of 16.
+static int batch_run(int ntiles, int grid) {
+  const long long even = ((long long)ntiles + grid - 1) / grid;
+  for (int run = kBatchRunMax; run > 1; run /= 2) {
+    const long long units = ((long long)ntiles + run - 1) / run;
+    const long long most = (units + grid - 1) / grid * run;
+    if (16 * most <= 17 * even) return run;
+  }
+  return 1;
+}
+
 template <class Pol, bool HLLD, int TY, bool BATCHED>
-static void launch_one(int stage, const Batch& b, const Member& m0, int parity, int grid, cudaStream_t s) {
+static void launch_one(int stage, const Batch& b, const Member& m0, int parity, int run, int grid, cudaStream_t s) {
   const size_t smem = Smem<Pol, TY>::total;
   if (stage == 1)
-    stage_kernel<Pol, 1, HLLD, TY, BATCHED><<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity);
+    stage_kernel<Pol, 1, HLLD, TY, BATCHED><<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run);
   else
-    stage_kernel<Pol, 2, HLLD, TY, BATCHED><<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity);
+    stage_kernel<Pol, 2, HLLD, TY, BATCHED><<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run);
 }
 
 template <class Pol, int TY>
@@ -108,20 +124,21 @@ static cudaError_t launch_stage_pol(int hlld, int stage, const Batch& b, const M
   if (b.ntiles <= 0) return cudaSuccess;
   const bool batched = single == nullptr;
   if (grid <= 0) grid = sm_count() * occ_pol_ty<Pol, TY>(hlld, batched);
-  const int units = batched ? (b.ntiles + kBatchRun - 1) / kBatchRun : b.ntiles;  // tiles or runs of tiles
+  const int run = batched ? batch_run(b.ntiles, grid) : 1;
+  const int units = (b.ntiles + run - 1) / run;  // runs of tiles
   if (grid > units) grid = units;
   static const Member empty = {};
   const Member& m0 = batched ? empty : *single;
   if (hlld) {
     if (batched)
-      launch_one<Pol, true, TY, true>(stage, b, m0, parity, grid, s);
+      launch_one<Pol, true, TY, true>(stage, b, m0, parity, run, grid, s);
     else
-      launch_one<Pol, true, TY, false>(stage, b, m0, parity, grid, s);
+      launch_one<Pol, true, TY, false>(stage, b, m0, parity, run, grid, s);
   } else {
     if (batched)
-      launch_one<Pol, false, TY, true>(stage, b, m0, parity, grid, s);
+      launch_one<Pol, false, TY, true>(stage, b, m0, parity, run, grid, s);
     else
-      launch_one<Pol, false, TY, false>(stage, b, m0, parity, grid, s);
+      launch_one<Pol, false, TY, false>(stage, b, m0, parity, run, grid, s);
   }
   return cudaGetLastError();
 }

@@ -432,10 +432,11 @@ __device__ __forceinline__ bool member_active(const Member& m, int p) {
 // BATCHED = false: one grid, passed by value as a kernel parameter (its
 // scalars are then constant-bank operands and its TMA descriptors live in
 // parameter space); `b` only supplies the tile count.  BATCHED = true: the
-// members of `b`, read from device memory per tile.
+// members of `b`, read from device memory per tile, handed out in runs of
+// `run` (a power of two) consecutive tiles.
 template <class Pol, int STAGE, bool HLLD, int TY, bool BATCHED>
 __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
-    stage_kernel(const __grid_constant__ Member m0, const Batch b, const int p) {
+    stage_kernel(const __grid_constant__ Member m0, const Batch b, const int p, const int run) {
   using S = typename Pol::S;
   using R = typename Pol::R;
   using G = Geo<TY>;
@@ -462,15 +463,15 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
   }
 
   // Tile order.  One grid: tile blockIdx.x, then every gridDim.x-th.  A
-  // batch: runs of kBatchRun consecutive tiles, run blockIdx.x, then
+  // batch: runs of `run` consecutive tiles, run blockIdx.x, then
   // every gridDim.x-th run -- consecutive tiles of a CTA then mostly share
   // a member, so its descriptor, control slot and step values are re-read
   // once per member run instead of once per tile, while members that stop
   // early still leave their tiles spread over all CTAs.
-  auto first_tile = [&]() { return BATCHED ? (int)blockIdx.x * kBatchRun : (int)blockIdx.x; };
+  auto first_tile = [&]() { return BATCHED ? (int)blockIdx.x * run : (int)blockIdx.x; };
   auto after = [&](int t) {
     if constexpr (BATCHED)
-      return (t + 1) % kBatchRun != 0 ? t + 1 : t + 1 + ((int)gridDim.x - 1) * kBatchRun;
+      return ((t + 1) & (run - 1)) != 0 ? t + 1 : t + 1 + ((int)gridDim.x - 1) * run;
     else
       return t + (int)gridDim.x;
   };

@@ -346,3 +346,24 @@ def test_per_size_tuned_plan_is_bit_identical(pmhd_lib):
             assert ms.steps == st.steps and ms.t == st.t, k
             assert (ms.degenerate, ms.nonphysical) == (st.degenerate, st.nonphysical), k
             np.testing.assert_array_equal(e.get_state(k), U, err_msg=f"member {k}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 149, 592, 2368, 2373])
+def test_every_run_length_covers_the_work_list(pmhd_lib, count):
+    """Work lists of one-tile members (8 x 8) around multiples of the SM count,
+    which hand the CTAs runs of 1, 2, 4 and 16 tiles: every member gets the
+    bits of its single-grid run."""
+    b0 = [0.7, 1.0, 1.3]
+    ref = []
+    for b in b0:
+        with pmhd_lib.Solver(nx=8, ny=8, precision="fp32", exact=True) as s:
+            s.init_problem(pmhd_lib.PROBLEM_ORSZAG_TANG, [b])
+            s.advance(max_steps=3)
+            ref.append(s.get_state())
+    ms = [pmhd_lib.member(8, 8, pmhd_lib.PROBLEM_ORSZAG_TANG, (b0[k % 3],), t_end=10.0) for k in range(count)]
+    with pmhd_lib.Ensemble(ms, precision="fp32", exact=True) as e:
+        e.advance(max_steps=3)
+        for k in range(count):
+            assert e.member_stats(k).steps == 3
+            np.testing.assert_array_equal(e.get_state(k), ref[k % 3])
