@@ -169,6 +169,11 @@ __device__ __forceinline__ void hancock_faces(HancockTileOf<Pol>& s, const Hanco
   }
 }
 
+template <int AX>
+struct AxisTag {
+  static constexpr int value = AX;
+};
+
 // Interface fluxes of the tile at (i0, j0): x-interface (r, c) = between
 // tile columns c-1 and c (c = 0..32) of tile row r; y-interface (r, c) =
 // between tile rows r-1 and r (r = 0..TYH) of tile column c.  Stored over
@@ -185,30 +190,42 @@ __device__ __forceinline__ void hancock_fluxes(HancockTileOf<Pol>& s, const Memb
   R* Gy = &s.f.Gy[0][0];
   const GlmK<R> gk = GlmK<R>::make(ch);
   for (int q = first; q < HT::NFX + HT::NGY; q += step) {
-    R a[NVAR], b[NVAR], F[NVAR];
     int st;
+    auto flux = [&](auto axis, const R* ha, const R* hb, R* out, int n_out) {  // faces at ha / hb, plane stride NB
+      constexpr int AX = decltype(axis)::value;
+      if constexpr (kLeanFlux<R>) {
+        return glm_flux_lean<R, AX, true>(
+            gk, HLLD, ph,
+            [&](R* a, R* b) {
+#pragma unroll
+              for (int k = 0; k < NVAR; k++) {
+                a[k] = ha[k * HT::NB];
+                b[k] = hb[k * HT::NB];
+              }
+            },
+            [&](int k, R f) { out[k * n_out] = f; });
+      } else {
+        R a[NVAR], b[NVAR], F[NVAR];
+#pragma unroll
+        for (int k = 0; k < NVAR; k++) {
+          a[k] = ha[k * HT::NB];
+          b[k] = hb[k * HT::NB];
+        }
+        const int code = PMHD_FAST_FLUX ? glm_flux_fast_cons<R, AX>(a, b, gk, HLLD, F, ph)
+                                        : glm_flux<R, AX>(a, b, ch, HLLD, F, ph);
+#pragma unroll
+        for (int k = 0; k < NVAR; k++) out[k * n_out] = F[k];
+        return code;
+      }
+    };
     if (q < HT::NFX) {
       const int r = q / (TX + 1), c = q % (TX + 1);
       const int bl = (r + 1) * BW + c, br = bl + 1;  // box cells left / right of the interface
-#pragma unroll
-      for (int k = 0; k < NVAR; k++) {
-        a[k] = s.H[1][k][bl];
-        b[k] = s.H[0][k][br];
-      }
-      st = PMHD_FAST_FLUX ? glm_flux_fast_cons<R, 0>(a, b, gk, HLLD, F, ph) : glm_flux<R, 0>(a, b, ch, HLLD, F, ph);
-#pragma unroll
-      for (int k = 0; k < NVAR; k++) Fx[k * HT::NFX + q] = F[k];
+      st = flux(AxisTag<0>{}, &s.H[1][0][bl], &s.H[0][0][br], Fx + q, HT::NFX);
     } else {
       const int g = q - HT::NFX, r = g / TX, c = g % TX;
       const int bb = r * BW + (c + 1), bt = bb + BW;  // box cells below / above
-#pragma unroll
-      for (int k = 0; k < NVAR; k++) {
-        a[k] = s.H[3][k][bb];
-        b[k] = s.H[2][k][bt];
-      }
-      st = PMHD_FAST_FLUX ? glm_flux_fast_cons<R, 1>(a, b, gk, HLLD, F, ph) : glm_flux<R, 1>(a, b, ch, HLLD, F, ph);
-#pragma unroll
-      for (int k = 0; k < NVAR; k++) Gy[k * HT::NGY + g] = F[k];
+      st = flux(AxisTag<1>{}, &s.H[3][0][bb], &s.H[2][0][bt], Gy + g, HT::NGY);
     }
     if (HLLD) {
       // Count each interface of the domain once: interface I (between

@@ -113,9 +113,11 @@ constexpr size_t align128(size_t b) { return (b + 127) & ~size_t(127); }
 // whose 16 K-register files then allow 96 registers a thread.  A 32 x 16
 // tile has 17 warps (5 / 4 / 4 / 4 per scheduler, so the same 96-register
 // cap with fewer warps), a 32 x 15 tile 16 warps at 128 registers.  At
-// 4096^2 (performance build) 32 x 19 runs mixed 5.91, fp64 2.42, fp32 6.68 G
-// zone-cycles/s against 5.25 / 2.20 / 6.04 at 32 x 16 and 5.90 / 2.28 / 6.69
-// at 32 x 15; it also recomputes the fewest halo interfaces and recoveries
+// 4096^2 (performance build) 32 x 19 runs mixed 5.91, fp32 6.68 G
+// zone-cycles/s against 5.25 / 6.04 at 32 x 16 and 5.90 / 6.69 at 32 x 15
+// (binary64 at 2048^2, with glm_flux_lean: 3.41 G at 32 x 19, 196 / 232 bytes of
+// spill stores in stage 1 / 2; glm_flux_fast's 520 / 552 bytes went to L2
+// because 211 KB of shared memory leave the L1 16 KB: 3.11 G); it also recomputes the fewest halo interfaces and recoveries
 // (2.08 interface solves and 1.34 recoveries per cell; 32 x 16: 2.09 / 1.41;
 // 32 x 8: 2.16 / 1.63).  32 x 4 tiles keep about the same threads per SM as
 // 32 x 8.  PMHD_NBUF / PMHD_MINB_R32 / PMHD_MINB_R64 override the 32 x 8
@@ -201,7 +203,7 @@ __device__ __forceinline__ void recover_cell(const typename Pol::S* U, typename 
   } else if (PMHD_FAST_FLUX) {
     // Performance build: one reciprocal of the density for the velocities.
     using S = typename Pol::S;
-    const S rho = vmax(U[RHO], rho_floor<S>());
+    const S rho = at_least(U[RHO], rho_floor<S>());
     const S inv = fast_rcp(rho);
     const S vx = U[MX] * inv, vy = U[MY] * inv, vz = U[MZ] * inv;
     const S bx = U[BX], by = U[BY], bz = U[BZ];
@@ -337,6 +339,65 @@ __device__ __forceinline__ int face_flux(const typename Pol::R* sP, bool checks,
     }
   }
   return glm_flux<R, 0, PMHD_FAST_FLUX != 0>(UL, UR, gk.ch, HLLD, F, ph);
+}
+
+// Performance build, binary64 faces: glm_flux_lean (binary32 faces fit their
+// registers with glm_flux_fast).
+template <class R>
+constexpr bool kLeanFlux = PMHD_FAST_FLUX != 0 && sizeof(R) == 8;
+
+// Face of one cell from its three stencil values along an axis (plane offsets
+// off[k], value stride `stride`, first value at q): the cell's right face, or
+// its left one (RIGHT = false).  recon_cell for one face: first order when
+// either face is unusable.  Re-reads the cell instead of holding both faces.
+template <class R, bool RIGHT>
+__device__ __forceinline__ void checked_face(const R* q, const int (&off)[NVAR], int stride, R* P) {
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < NVAR; k++) {
+    const R c = q[off[k] + stride];
+    const R s = minmod(c - q[off[k]], q[off[k] + 2 * stride] - c);
+    const R l = c - (R)0.5 * s, r = c + (R)0.5 * s;
+    if (k == RHO) ok = ok && !(l <= rho_floor<R>()) && !(r <= rho_floor<R>());
+    if (k == EN) ok = ok && !(l <= p_floor<R>()) && !(r <= p_floor<R>());
+    ok = ok && vfinite(l) && vfinite(r);
+    P[k] = RIGHT ? r : l;
+  }
+  if (!ok) {
+#pragma unroll
+    for (int k = 0; k < NVAR; k++) P[k] = q[off[k] + stride];
+  }
+}
+
+// face_flux through glm_flux_lean, from the tile's primitives (also at first
+// order, whose faces are the cell values); flux slots leave through
+// emit(slot, value), in x-normal order.
+template <class R, bool HLLD, int TC, class Emit>
+__device__ __forceinline__ int face_flux_lean(const R* sP, bool checks, int base, int stride, int o1, int o2, int o5,
+                                              int o6, int muscl, const GlmK<R>& gk, const Phys<R>& ph, Emit&& emit) {
+  const int off[NVAR] = {0, o1, o2, 3 * TC, 4 * TC, o5, o6, 7 * TC, 8 * TC};
+  auto load = [&](R* Pa, R* Pb) {
+    const R* q = sP + base;
+    if (muscl && !checks) {
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) {
+        const R P0 = q[off[k] + stride], P1 = q[off[k] + 2 * stride];
+        const R d1 = P1 - P0;
+        Pa[k] = P0 + (R)0.5 * minmod_fast(P0 - q[off[k]], d1);
+        Pb[k] = P1 - (R)0.5 * minmod_fast(d1, q[off[k] + 3 * stride] - P1);
+      }
+    } else if (muscl) {
+      checked_face<R, true>(q, off, stride, Pa);
+      checked_face<R, false>(q + stride, off, stride, Pb);
+    } else {
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) {
+        Pa[k] = q[off[k] + stride];
+        Pb[k] = q[off[k] + 2 * stride];
+      }
+    }
+  };
+  return glm_flux_lean<R, 0, false>(gk, HLLD, ph, load, emit);
 }
 
 // Per-member step values (uniform for all tiles of a member in one launch).
@@ -542,7 +603,8 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
     }
 
     // ---- recovery, once per tile cell (halo corners are never used) -------
-    // First order needs no primitives: the conserved states are staged.
+    // First order needs no primitives (but for the lean binary64 flux): the
+    // conserved states are staged.
     bool usable = true;  // performance build: this thread's cells (cell_usable_fast)
     for (int q = tid; q < TC; q += NT) {
       const int cx = q % HX, cy = q / HX;
@@ -550,7 +612,7 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
       S U9[NVAR], P9[NVAR];
 #pragma unroll
       for (int k = 0; k < NVAR; k++) U9[k] = sU[k * TC + q];
-      if (m.muscl) {
+      if (kLeanFlux<R> || m.muscl) {
         recover_cell<Pol>(U9, P9, phS);
       } else {
 #pragma unroll
@@ -605,21 +667,33 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
       const int stride = axis ? HX : 1;
       const int o1 = (axis ? 2 : 1) * TC, o2 = (axis ? 1 : 2) * TC;
       const int o5 = (axis ? 6 : 5) * TC, o6 = (axis ? 5 : 6) * TC;
-      R F[NVAR];
-      const int st = face_flux<Pol, HLLD, TC>(sP, checks, base, stride, o1, o2, o5, o6, m.muscl, GlmK<R>::make(v.ch), phR, F);
-      R* out = axis ? sGy : sFx;
-      const int n_out = axis ? GYN : FXN;
-      const int item = axis ? fy * TX + fx : fy * (TX + 1) + fx;
-      const int p1 = axis ? 2 : 1, p2 = axis ? 1 : 2, p5 = axis ? 6 : 5, p6 = axis ? 5 : 6;
-      out[0 * n_out + item] = F[0];
-      out[p1 * n_out + item] = F[1];
-      out[p2 * n_out + item] = F[2];
-      out[3 * n_out + item] = F[3];
-      out[4 * n_out + item] = F[4];
-      out[p5 * n_out + item] = F[5];
-      out[p6 * n_out + item] = F[6];
-      out[7 * n_out + item] = F[7];
-      out[8 * n_out + item] = F[8];
+      int st;
+      if constexpr (kLeanFlux<R>) {
+        R* out = axis ? sGy + fy * TX + fx : sFx + fy * (TX + 1) + fx;
+        const int n_out = axis ? GYN : FXN;
+        auto emit = [&](int k, R f) {  // flux slot k of the x-ordered problem
+          const int q = k == 1 ? (axis ? 2 : 1) : k == 2 ? (axis ? 1 : 2) : k == 5 ? (axis ? 6 : 5) : k == 6 ? (axis ? 5 : 6) : k;
+          out[q * n_out] = f;
+        };
+        st = face_flux_lean<R, HLLD, TC>(sP, checks, base, stride, o1, o2, o5, o6, m.muscl, GlmK<R>::make(v.ch), phR,
+                                         emit);
+      } else {
+        R F[NVAR];
+        st = face_flux<Pol, HLLD, TC>(sP, checks, base, stride, o1, o2, o5, o6, m.muscl, GlmK<R>::make(v.ch), phR, F);
+        R* out = axis ? sGy : sFx;
+        const int n_out = axis ? GYN : FXN;
+        const int item = axis ? fy * TX + fx : fy * (TX + 1) + fx;
+        const int p1 = axis ? 2 : 1, p2 = axis ? 1 : 2, p5 = axis ? 6 : 5, p6 = axis ? 5 : 6;
+        out[0 * n_out + item] = F[0];
+        out[p1 * n_out + item] = F[1];
+        out[p2 * n_out + item] = F[2];
+        out[3 * n_out + item] = F[3];
+        out[4 * n_out + item] = F[4];
+        out[p5 * n_out + item] = F[5];
+        out[p6 * n_out + item] = F[6];
+        out[7 * n_out + item] = F[7];
+        out[8 * n_out + item] = F[8];
+      }
       if (HLLD && ((axis ? fy : fx) >= 1 || (axis ? j0 : i0) == 0)) {
         acc.n_deg += (st == HLLD_FALLBACK_DEGENERATE);
         acc.n_np += (st == HLLD_FALLBACK_NONPHYSICAL);
