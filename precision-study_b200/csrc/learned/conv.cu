@@ -7,19 +7,13 @@
 // (dx+1): out(y, x) = sum_t W[t] x(y+dy, x+dx) (cross-correlation).
 //
 // Implicit GEMM.  Forward / backward-data: M = 128 output pixels x N = c_out
-// channels, K = 9 taps x c_in channels.  Row kernels (width a multiple of
-// 128, height of 8): a row tile's input is staged once, each tap's operand
-// is a shifted descriptor into it, one thread issues 8 rows x 9 * c_in / 16
-// tcgen05.mma, eight warps run the epilogue -- one CTA per tile, or (from
-// two tiles per SM) a persistent CTA per SM whose producer, MMA and
-// epilogue warps pipeline the tiles.  Gather kernel (other shapes):
-// one CTA per 128 pixels gathers the 9 shifted copies of its pixels' input
-// vectors (periodic wrap) into K-major tiles, one thread issues 9 * c_in / 16
-// tcgen05.mma, the four warps read the 128 x N accumulator back with
-// tcgen05.ld and run the epilogue.  Weight gradient: D[(t, c_in)][c_out] =
-// sum over pixels of x(p + tap) dz(p)^T, K = pixels: blocks of 8 pixels x 8
-// channels are transposed in registers into K-major tiles, three M = 128
-// tiles accumulate over 64-pixel chunks, CTAs sum with fp32 atomics.
+// channels, K = 9 taps x c_in channels.  A persistent CTA per SM walks tiles of
+// 8 image rows x 128 pixels; a tile's input is staged once, each tap's operand
+// is a shifted descriptor into it, and producer, MMA and epilogue warps pipeline
+// the tiles.  Weight gradient: D[(row, c_in)][(row, c_out)] = sum over pixels of
+// x(p + tap) dz(p)^T, K = pixels; both operands are channel-major (MN-major) as
+// NHWC has them, staged once per tile of 8 rows x 64 pixels, and one MMA covers
+// three vertical taps of two output rows; CTAs sum with fp32 atomics.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -62,396 +56,195 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return s + z * s * (1.0f - s) * (kGeluA + 3.0f * kGeluB * z * z);
 }
 
+// Two 16-byte vectors to / from consecutive addresses: one 32-byte access (a full
+// L2 sector) when the buffers allow it (`wide`: 32-byte aligned), else two.
+__device__ __forceinline__ void store32(void* p, const uint4& a, const uint4& b, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+  } else {
+    static_cast<uint4*>(p)[0] = a;
+    static_cast<uint4*>(p)[1] = b;
+  }
+}
+__device__ __forceinline__ void load32(const void* p, uint4& a, uint4& b, bool wide) {
+  if (wide) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
+  } else {
+    a = static_cast<const uint4*>(p)[0];
+    b = static_cast<const uint4*>(p)[1];
+  }
+}
+
 __device__ __forceinline__ int wrap(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 
-__device__ __forceinline__ uint32_t word_of(const uint4& v, int i) {
-  return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
-}
-
-// Row `ch` of the 8 x 8 bf16 transpose of v[0..7] (v[q] = 8 channels of
-// pixel q): the 8 pixels' values of channel ch, pixel q in halfword q.
-__device__ __forceinline__ uint4 transpose_row(const uint4 (&v)[8], int ch) {
-  const uint32_t sel = (ch & 1) ? 0x7632u : 0x5410u;
-  const int wi = ch >> 1;
-  uint4 r;
-  r.x = __byte_perm(word_of(v[0], wi), word_of(v[1], wi), sel);
-  r.y = __byte_perm(word_of(v[2], wi), word_of(v[3], wi), sel);
-  r.z = __byte_perm(word_of(v[4], wi), word_of(v[5], wi), sel);
-  r.w = __byte_perm(word_of(v[6], wi), word_of(v[7], wi), sel);
-  return r;
-}
-
-// Bounded wait for the MMA batch; on expiry record the error and wait once
-// more (bounded) so tensor memory is not released under a running MMA.
-__device__ __forceinline__ bool wait_mma(uint64_t* bar, uint32_t parity, int* err) {
-  bool ok = mbar_wait_bounded(bar, parity, kWaitPolls);
-  ok = __all_sync(0xffffffffu, ok);
-  if (!ok) {
-    if ((threadIdx.x & 31) == 0) atomicExch(err, PMHD_LEARNED_ERR_TIMEOUT);
-    mbar_wait_bounded(bar, parity, kWaitPolls);
-  }
-  return ok;
-}
-
-// Epilogue of one output pixel p from its CO fp32 accumulators; `bias` is
-// the CTA's 16-byte-aligned shared copy (unused by CONV_DGELU).
+// Epilogue of 16 channels (from c0) of one output pixel p from their fp32
+// accumulators; `bias` is the CTA's 16-byte-aligned shared copy (unused by
+// CONV_DGELU); wide: see store32.
 template <int CO, int EPI>
-__device__ __forceinline__ void epilogue(const float (&acc)[CO], long long p, const float* __restrict__ bias,
-                                         const __nv_bfloat16* __restrict__ zprev, void* __restrict__ out0,
-                                         void* __restrict__ out1) {
+__device__ __forceinline__ void epilogue16(const float (&acc)[16], int c0, long long p, const float* __restrict__ bias,
+                                           const __nv_bfloat16* __restrict__ zprev, void* __restrict__ out0,
+                                           void* __restrict__ out1, bool wide) {
+  float bb[16];
+  if (EPI != CONV_DGELU) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float4 b = reinterpret_cast<const float4*>(bias + c0)[q];
+      bb[4 * q] = b.x, bb[4 * q + 1] = b.y, bb[4 * q + 2] = b.z, bb[4 * q + 3] = b.w;
+    }
+  }
+  auto vec = [](const uint32_t* w) { return make_uint4(w[0], w[1], w[2], w[3]); };
   if (EPI == CONV_GELU) {
-    __nv_bfloat16* z = static_cast<__nv_bfloat16*>(out0) + p * CO;
-    __nv_bfloat16* a = static_cast<__nv_bfloat16*>(out1) + p * CO;
+    uint32_t zb[8], ab[8];
 #pragma unroll
-    for (int c8 = 0; c8 < CO / 8; c8++) {
-      __align__(16) __nv_bfloat162 zb[4], ab[4];
-      const float4 b0 = reinterpret_cast<const float4*>(bias)[c8 * 2];
-      const float4 b1 = reinterpret_cast<const float4*>(bias)[c8 * 2 + 1];
-      const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float z0 = acc[c8 * 8 + 2 * q] + bb[2 * q];
-        const float z1 = acc[c8 * 8 + 2 * q + 1] + bb[2 * q + 1];
-        zb[q] = __floats2bfloat162_rn(z0, z1);
-        ab[q] = __floats2bfloat162_rn(gelu(z0), gelu(z1));
-      }
-      *reinterpret_cast<uint4*>(z + c8 * 8) = *reinterpret_cast<const uint4*>(zb);
-      *reinterpret_cast<uint4*>(a + c8 * 8) = *reinterpret_cast<const uint4*>(ab);
+    for (int q = 0; q < 8; q++) {
+      const float z0 = acc[2 * q] + bb[2 * q];
+      const float z1 = acc[2 * q + 1] + bb[2 * q + 1];
+      const __nv_bfloat162 z2 = __floats2bfloat162_rn(z0, z1), a2 = __floats2bfloat162_rn(gelu(z0), gelu(z1));
+      zb[q] = *reinterpret_cast<const uint32_t*>(&z2);
+      ab[q] = *reinterpret_cast<const uint32_t*>(&a2);
     }
+    store32(static_cast<__nv_bfloat16*>(out0) + p * CO + c0, vec(zb), vec(zb + 4), wide);
+    store32(static_cast<__nv_bfloat16*>(out1) + p * CO + c0, vec(ab), vec(ab + 4), wide);
   } else if (EPI == CONV_LINEAR) {
-    float* o = static_cast<float*>(out0) + p * CO;
+    uint32_t v[16];
 #pragma unroll
-    for (int c4 = 0; c4 < CO / 4; c4++) {
-      const float4 b = reinterpret_cast<const float4*>(bias)[c4];
-      float4 v;
-      v.x = acc[c4 * 4 + 0] + b.x;
-      v.y = acc[c4 * 4 + 1] + b.y;
-      v.z = acc[c4 * 4 + 2] + b.z;
-      v.w = acc[c4 * 4 + 3] + b.w;
-      *reinterpret_cast<float4*>(o + c4 * 4) = v;
-    }
+    for (int q = 0; q < 16; q++) v[q] = __float_as_uint(acc[q] + bb[q]);
+    float* o = static_cast<float*>(out0) + p * CO + c0;
+    store32(o, vec(v), vec(v + 4), wide);
+    store32(o + 8, vec(v + 8), vec(v + 12), wide);
   } else {
-    const __nv_bfloat16* zp = zprev + p * CO;
-    __nv_bfloat16* d = static_cast<__nv_bfloat16*>(out0) + p * CO;
+    uint4 za, zc;
+    load32(zprev + p * CO + c0, za, zc, wide);
+    const uint32_t zw[8] = {za.x, za.y, za.z, za.w, zc.x, zc.y, zc.z, zc.w};
+    uint32_t db[8];
 #pragma unroll
-    for (int c8 = 0; c8 < CO / 8; c8++) {
-      const uint4 zv = *reinterpret_cast<const uint4*>(zp + c8 * 8);
-      const __nv_bfloat16* zs = reinterpret_cast<const __nv_bfloat16*>(&zv);
-      __align__(16) __nv_bfloat16 db[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) db[q] = __float2bfloat16_rn(acc[c8 * 8 + q] * gelu_grad(__bfloat162float(zs[q])));
-      *reinterpret_cast<uint4*>(d + c8 * 8) = *reinterpret_cast<const uint4*>(db);
+    for (int q = 0; q < 8; q++) {
+      const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&zw[q]));
+      const __nv_bfloat162 d = __floats2bfloat162_rn(acc[2 * q] * gelu_grad(z.x), acc[2 * q + 1] * gelu_grad(z.y));
+      db[q] = *reinterpret_cast<const uint32_t*>(&d);
     }
+    store32(static_cast<__nv_bfloat16*>(out0) + p * CO + c0, vec(db), vec(db + 4), wide);
   }
 }
 
-// B operand: the weights [CO][9 CG], K-groups of 8 (16-byte vectors) at
-// kLboB = CO * 16; thread t of nt.
-template <int CG, int CO>
+// B operand: for each horizontal shift dx of the input (dx + 1 = 0, 1, 2) and
+// 8-channel group, the 16-byte vectors of 3 CO weights: those that take the input
+// row to output rows one above (shift dy = 1), level and one below it; the
+// backward pass mirrors the taps.  Thread t of nt.
+template <int CG, int CO, int EPI>
 __device__ __forceinline__ void stage_weights(unsigned char* sB, const __nv_bfloat16* __restrict__ wt, int t,
                                               int nt) {
-  constexpr int K = 9 * CG;
+  constexpr int K = 9 * CG, NG = CG / 8;
   for (int c = t; c < CO * (K / 8); c += nt) {
-    const int n = c / (K / 8), g = c - n * (K / 8);
+    const int n = c / (K / 8), g = c - n * (K / 8), tap = g / NG;
+    const int sgn = EPI == CONV_DGELU ? -1 : 1, dy = sgn * (tap / 3 - 1), dx = sgn * (tap % 3 - 1);
     const uint4 v = *reinterpret_cast<const uint4*>(wt + (size_t)n * K + g * 8);
-    *reinterpret_cast<uint4*>(sB + n * 16 + g * CO * 16) = v;
+    *reinterpret_cast<uint4*>(sB + (((dx + 1) * NG + g % NG) * 3 * CO + (1 - dy) * CO + n) * 16) = v;
   }
 }
 
-template <int CG, int CO>
-struct ConvSmem {
-  static constexpr int K = 9 * CG;
-  static constexpr uint32_t kATap = 128u * CG * 2u;  // bytes of one tap tile
-  static constexpr uint32_t kLboA = 128u * 16u;      // K-group stride of A
-  static constexpr uint32_t kBytesB = (uint32_t)CO * K * 2u;
-  static constexpr uint32_t kLboB = (uint32_t)CO * 16u;
-  static constexpr uint32_t kOffB = 9u * kATap;
-  static constexpr uint32_t kOffBar = kOffB + kBytesB;
-  static constexpr uint32_t kBytes = kOffBar + 16u;
-};
-
-// EPI: CONV_GELU   out0 = z (bf16), out1 = gelu(z) (bf16), z = acc + bias
-//      CONV_LINEAR out0 = acc + bias (fp32)
-//      CONV_DGELU  out0 = acc * gelu'(zprev) (bf16); taps mirrored (the
-//                  transposed convolution of the backward pass)
-template <int CG, int CO, int EPI>
-__global__ void __launch_bounds__(128) conv3x3_kernel(const __nv_bfloat16* __restrict__ x,
-                                                      const __nv_bfloat16* __restrict__ wt,
-                                                      const float* __restrict__ bias,
-                                                      const __nv_bfloat16* __restrict__ zprev, int batch, int h,
-                                                      int w, void* __restrict__ out0, void* __restrict__ out1,
-                                                      int* __restrict__ err) {
-  using S = ConvSmem<CG, CO>;
-  constexpr uint32_t kCols = umma::tmem_cols(CO);
-  extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* sA = smem;
-  unsigned char* sB = smem + S::kOffB;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kOffBar + 8);
-  __shared__ __align__(16) float sbias[CO];
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const long long P = (long long)batch * h * w;
-  const long long p0 = (long long)blockIdx.x * 128;
-  if (tid < CO) sbias[tid] = EPI == CONV_DGELU ? 0.0f : bias[tid];
-
-  if (warp == 0) {
-    umma::tmem_alloc(tslot, kCols);
-    umma::tmem_relinquish();
-  }
-  if (tid == 0) {
-    mbar_init(bar, 1);
-    fence_barrier_init();
-  }
-  stage_weights<CG, CO>(sB, wt, tid, 128);
-  // A operand: for each tap, the 128 pixels' shifted input vectors.
-  for (int c = tid; c < 9 * 128 * (CG / 8); c += 128) {
-    const int g = c % (CG / 8);
-    const int m = (c / (CG / 8)) % 128;
-    const int t = c / (128 * (CG / 8));
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    const long long p = p0 + m;
-    if (p < P) {
-      const int x0 = (int)(p % w);
-      const long long r = p / w;
-      const int y0 = (int)(r % h);
-      const long long b = r / h;
-      int dy = t / 3 - 1, dx = t % 3 - 1;
-      if (EPI == CONV_DGELU) {
-        dy = -dy;
-        dx = -dx;
-      }
-      const int yy = wrap(y0 + dy, h), xx = wrap(x0 + dx, w);
-      v = *reinterpret_cast<const uint4*>(x + ((b * h + yy) * (long long)w + xx) * CG + g * 8);
-    }
-    *reinterpret_cast<uint4*>(sA + t * S::kATap + m * 16 + g * S::kLboA) = v;
-  }
-  fence_proxy_async_smem();
-  umma::fence_before_sync();
-  __syncthreads();
-  umma::fence_after_sync();
-  const uint32_t tmem = *tslot;
-  if (tid == 0) {
-    constexpr uint32_t idesc = umma::idesc_bf16(128, CO, false, false);
-    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-#pragma unroll 1
-    for (int t = 0; t < 9; t++)
-#pragma unroll
-      for (int kc = 0; kc < CG / 16; kc++) {
-        const uint64_t da = umma::desc(a0 + t * S::kATap + kc * 2 * S::kLboA, S::kLboA, 128);
-        const uint64_t db = umma::desc(b0 + (t * (CG / 8) + kc * 2) * S::kLboB, S::kLboB, 128);
-        umma::mma_bf16(tmem, da, db, idesc, (t | kc) ? 1u : 0u);
-      }
-    umma::commit(bar);
-  }
-  __syncwarp();
-  const bool ok = wait_mma(bar, 0, err);
-  umma::fence_after_sync();
-  if (ok) {
-    float acc[CO];
-#pragma unroll
-    for (int c8 = 0; c8 < CO / 8; c8++) umma::ld8(tmem + ((uint32_t)(warp * 32) << 16) + c8 * 8, acc + c8 * 8);
-    const long long p = p0 + tid;
-    if (p < P) epilogue<CO, EPI>(acc, p, sbias, zprev, out0, out1);
-  }
-  umma::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) {
-    umma::fence_after_sync();
-    umma::tmem_dealloc(tmem, kCols);
-  }
+// 16-byte asynchronous copy; the form with `take` zero-fills when it is false.
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void* src, bool take) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(take ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 constexpr int kRowPix = 128;               // output pixels of a row segment (M)
 constexpr int kRows = 8;                   // output rows per tile
 constexpr int kRowPitch = kRowPix + 2;     // staged pixels per input row
-constexpr int kRowThreads = 256;
-constexpr uint32_t kRowLboA = (uint32_t)(kRows + 2) * kRowPitch * 16u;  // channel-group stride of A
 
-template <int CG, int CO>
-struct RowSmem {
-  static constexpr int K = 9 * CG;
-  static constexpr uint32_t kBytesA = (uint32_t)(CG / 8) * kRowLboA;
-  static constexpr uint32_t kOffB = (kBytesA + 127u) & ~127u;
-  static constexpr uint32_t kBytesB = (uint32_t)CO * K * 2u;
-  static constexpr uint32_t kOffBar = kOffB + kBytesB;
-  static constexpr uint32_t kBytes = kOffBar + 16u;
-  // Shared memory requested per CTA: at least enough that no more CTAs fit
-  // on an SM (228 KB) than its 512 tensor-memory columns hold; eight CTAs of
-  // 256 threads are the thread limit anyway.
-  static constexpr uint32_t kTmemCols = umma::tmem_cols(kRows * CO);
-  static constexpr uint32_t kMaxCtas = 512u / kTmemCols;
-  static constexpr uint32_t kMinBytes = kMaxCtas >= 8u ? 0u : (228u * 1024u) / (kMaxCtas + 1u) + 1024u;
-  static constexpr uint32_t kLaunchBytes = kBytes > kMinBytes ? kBytes : kMinBytes;
-};
-
-// A row tile: image bb, output rows y0 .. y0 + kRows - 1, pixels x0 .. x0 + 127.
+// A row tile: image bb, output rows y0 .. y0 + kRows - 1, pixels x0 .. x0 + 127,
+// of which `rows` rows and `pix` pixels lie in the image.
 struct RowTile {
   long long bb;
-  int y0, x0;
+  int y0, x0, rows, pix;
 };
+template <int ROWS, int PIX>
 __device__ __forceinline__ RowTile row_tile(long long tile, int h, int w) {
-  const int segs = w / kRowPix, rblocks = h / kRows;
+  const int segs = (w + PIX - 1) / PIX, rblocks = (h + ROWS - 1) / ROWS;
   RowTile t;
-  t.x0 = (int)(tile % segs) * kRowPix;
-  t.y0 = (int)((tile / segs) % rblocks) * kRows;
+  t.x0 = (int)(tile % segs) * PIX;
+  t.y0 = (int)((tile / segs) % rblocks) * ROWS;
   t.bb = tile / ((long long)segs * rblocks);
+  t.rows = h - t.y0 < ROWS ? h - t.y0 : ROWS;
+  t.pix = w - t.x0 < PIX ? w - t.x0 : PIX;
   return t;
 }
 
-// A operand of a row tile: input rows y0 - 1 .. y0 + kRows, pixels
-// x0 - 1 .. x0 + 128 (periodic), one 16-byte channel group per item
-// (consecutive items are consecutive 16-byte words of the NHWC input), by
-// asynchronous copies from thread t of nt; the caller waits for them.
-template <int CG>
-__device__ __forceinline__ void stage_row_tile(unsigned char* sA, const __nv_bfloat16* __restrict__ x,
-                                               const RowTile& rt, int h, int w, int t, int nt) {
-  for (int c = t; c < (kRows + 2) * kRowPitch * (CG / 8); c += nt) {
-    const int g = c % (CG / 8);
-    const int px = (c / (CG / 8)) % kRowPitch;
-    const int r = c / ((CG / 8) * kRowPitch);
-    const int yy = wrap(rt.y0 - 1 + r, h), xx = wrap(rt.x0 - 1 + px, w);
-    const uint32_t dst = smem_u32(sA + g * kRowLboA + (r * kRowPitch + px) * 16);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst),
-                 "l"(x + ((rt.bb * h + yy) * (long long)w + xx) * CG + g * 8)
-                 : "memory");
+// Staged row r of a row tile (input row y0 - 1 + r, pixels x0 - 1 .. x0 + pix,
+// periodic) by one warp: 16-byte chunks of staged pixel s at dst + s * 2 CG,
+// swizzled (umma::swz).  Consecutive lanes copy consecutive 16-byte words.  ZERO:
+// pixels up to PIX + 1 and rows outside the tile are zero-filled; else they are
+// left alone (they feed accumulator rows that are never read).
+template <int CG, int PIX, bool ZERO>
+__device__ __forceinline__ void stage_halo_row(uint32_t dst, const __nv_bfloat16* __restrict__ x, const RowTile& rt,
+                                               int r, int h, int w, int lane) {
+  constexpr int NG = CG / 8, PER = 32 / NG;  // chunks a pixel, pixels a pass of the warp (512 bytes)
+  const bool row_in = r <= rt.rows + 1;
+  if (!ZERO && !row_in) return;
+  const int yy = row_in ? wrap(rt.y0 - 1 + r, h) : 0;
+  const __nv_bfloat16* row = x + (rt.bb * h + yy) * (long long)w * CG + lane % NG * 8;
+  const int last = row_in ? rt.pix + 1 : -1;  // last staged pixel that is used
+  dst = umma::swz<2 * CG>(dst + lane * 16);   // the swizzle does not see steps of 512 bytes
+#pragma unroll
+  for (int i = 0; i < (PIX + 2 + PER - 1) / PER; i++) {
+    const int s = lane / NG + i * PER;
+    const int col = wrap(rt.x0 - 1 + s, w);
+    if (ZERO) {
+      if (s < PIX + 2) cp16_or_zero(dst + i * 512, row + (s <= last ? (long long)col * CG : 0), s <= last);
+    } else {
+      if (s <= last) cp16(dst + i * 512, row + (long long)col * CG);
+    }
   }
 }
 
-// The row tile's MMAs, issued by one thread: for output row r and tap
-// (dy, dx) (mirrored for CONV_DGELU) the A operand is the staged tile seen
-// from pixel 1 + dx of staged row r + 1 + dy -- a shift of the descriptor's
-// start address; accumulators of row r at d0 + r * CO.
-template <int CG, int CO, int EPI>
-__device__ __forceinline__ void issue_row_mmas(uint32_t a0, uint32_t b0, uint32_t d0) {
-  constexpr uint32_t idesc = umma::idesc_bf16(128, CO, false, false);
-  constexpr uint32_t kLboB = (uint32_t)CO * 16u;
+// The row tile's MMAs, issued by one thread.  Staged input row r, shifted by dx
+// pixels (a shift of the descriptor's start address), feeds output rows r - 2,
+// r - 1 and r of the tile, whose accumulators are neighbours in tensor memory
+// (row o at d0 + o * CO): one MMA of N = 3 CO against the three vertical taps'
+// weights, less at the tile's first and last rows.  The first MMA on an output
+// row is its own (it does not accumulate).  A small MMA is bound by reading its
+// 4 KB of A from shared memory whatever N is (70 cycles at N = 32 and at 64,
+// measured without swizzle), so 68 MMAs of N <= 3 CO a tile of 8 rows at 32
+// channels take half the time of 144 of N = CO (8 x 512^2 layer: 142 -> 131 us a
+// call).
+template <int CG, int CO>
+__device__ __forceinline__ void issue_row_mmas(uint32_t a0, uint32_t b0, uint32_t d0, int rows) {
+  constexpr uint32_t kLboB = 3u * (uint32_t)CO * 16u;
+  const uint64_t a = umma::desc(a0, 16, 16 * CG, CG == 32 ? umma::kSwizzle64 : umma::kSwizzle32);
+  const uint64_t b = umma::desc(b0, kLboB, 128, umma::kNoSwizzle);
+  const uint32_t a_hi = umma::desc_hi(a), b_hi = umma::desc_hi(b), b_lo = umma::desc_lo(b);
+  uint32_t a_lo = umma::desc_lo(a);
+  // idesc of n blocks of CO columns.
+  auto idesc = [](int n) { return umma::idesc_bf16(128, 0, false, false) + ((uint32_t)(n * CO >> 3) << 17); };
 #pragma unroll 1
-  for (int r = 0; r < kRows; r++)
-#pragma unroll 1
-    for (int t = 0; t < 9; t++) {
-      int dy = t / 3 - 1, dx = t % 3 - 1;
-      if (EPI == CONV_DGELU) {
-        dy = -dy;
-        dx = -dx;
-      }
-      const uint32_t at = a0 + (uint32_t)(((r + 1 + dy) * kRowPitch + 1 + dx) * 16);
+  for (int r = 0; r < rows + 2; r++, a_lo += kRowPitch * CG / 8) {
+    const int lo = r < 2 ? 0 : r - 2, hi = r < rows ? r : rows - 1;  // output rows lo .. hi
+    const uint32_t skip = (uint32_t)((lo - (r - 2)) * CO);            // weight blocks before row lo's
+    const uint32_t d = d0 + (uint32_t)(lo * CO);
+    const bool fresh = r < rows;  // row r has no accumulator yet
+#pragma unroll
+    for (int dx = 0; dx < 3; dx++)
 #pragma unroll
       for (int kc = 0; kc < CG / 16; kc++) {
-        const uint64_t da = umma::desc(at + kc * 2 * kRowLboA, kRowLboA, 128);
-        const uint64_t db = umma::desc(b0 + (t * (CG / 8) + kc * 2) * kLboB, kLboB, 128);
-        umma::mma_bf16(d0 + (uint32_t)(r * CO), da, db, idesc, (t | kc) ? 1u : 0u);
+        const uint32_t al = a_lo + dx * (CG / 8) + kc * 2;
+        const uint32_t bl = b_lo + (dx * (CG / 8) + kc * 2) * (kLboB / 16) + skip;
+        if (dx + kc == 0 && fresh) {
+          if (r > 0) umma::mma_bf16(d, al, a_hi, bl, b_hi, idesc(hi - lo), 1u);
+          umma::mma_bf16(d0 + (uint32_t)(r * CO), al, a_hi, bl + (uint32_t)((hi - lo) * CO), b_hi, idesc(1), 0u);
+        } else {
+          umma::mma_bf16(d, al, a_hi, bl, b_hi, idesc(hi - lo + 1), 1u);
+        }
       }
-    }
-}
-
-// Reads a row tile's accumulators back (tensor-memory columns from tbase)
-// and runs the epilogue: warp `warp` of `nwarps` owns lane quarter warp % 4
-// (pixels 32 q .. 32 q + 31) of rows warp / 4, warp / 4 + nwarps / 4, ...
-template <int CO, int EPI>
-__device__ __forceinline__ void drain_row_tile(uint32_t tbase, int warp, int lane, int nwarps, const RowTile& rt,
-                                               int h, int w, const float* __restrict__ sbias,
-                                               const __nv_bfloat16* __restrict__ zprev, void* __restrict__ out0,
-                                               void* __restrict__ out1) {
-  const int q = warp & 3;
-  for (int r = warp >> 2; r < kRows; r += nwarps / 4) {
-    float acc[CO];
-#pragma unroll
-    for (int c8 = 0; c8 < CO / 8; c8++)
-      umma::ld8(tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)(r * CO + c8 * 8), acc + c8 * 8);
-    const long long p = (rt.bb * h + rt.y0 + r) * (long long)w + rt.x0 + q * 32 + lane;
-    epilogue<CO, EPI>(acc, p, sbias, zprev, out0, out1);
   }
 }
-
-// Row kernel (forward / backward-data when the width is a multiple of 128
-// and the height of 8), one CTA of 8 warps per row tile of kRows image rows
-// x 128 pixels.  It stages the (kRows + 2) x 130 input pixels around them
-// once (periodic wrap), channel-group-interleaved: group g of 8 channels at
-// g * kRowLboA, then row, then pixel at 16 bytes -- the K-major no-swizzle
-// layout of an M = 128 operand whose rows are pixels, so the nine taps need
-// no copies (issue_row_mmas).  Accumulators: 128 lanes x CO columns per row,
-// kRows rows side by side in tensor memory.  (Measured at batch 8 x 512^2:
-// 8, 4 and 2 rows per CTA -- two to four CTAs per SM -- run equally fast.)
-template <int CG, int CO, int EPI>
-__global__ void __launch_bounds__(kRowThreads) conv3x3_rows_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                   const __nv_bfloat16* __restrict__ wt,
-                                                                   const float* __restrict__ bias,
-                                                                   const __nv_bfloat16* __restrict__ zprev,
-                                                                   int batch, int h, int w,
-                                                                   void* __restrict__ out0, void* __restrict__ out1,
-                                                                   int* __restrict__ err) {
-  using S = RowSmem<CG, CO>;
-  constexpr uint32_t kCols = S::kTmemCols;
-  extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* sA = smem;
-  unsigned char* sB = smem + S::kOffB;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kOffBar + 8);
-  __shared__ __align__(16) float sbias[CO];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const RowTile rt = row_tile(blockIdx.x, h, w);
-  (void)batch;
-
-  if (warp == 0) {
-    umma::tmem_alloc(tslot, kCols);
-    umma::tmem_relinquish();
-  }
-  if (tid == 0) {
-    mbar_init(bar, 1);
-    fence_barrier_init();
-  }
-  if (tid < CO) sbias[tid] = EPI == CONV_DGELU ? 0.0f : bias[tid];
-  stage_weights<CG, CO>(sB, wt, tid, kRowThreads);
-  stage_row_tile<CG>(sA, x, rt, h, w, tid, kRowThreads);
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  fence_proxy_async_smem();
-  umma::fence_before_sync();
-  __syncthreads();
-  umma::fence_after_sync();
-  const uint32_t tmem = *tslot;
-  if (tid == 0) {
-    issue_row_mmas<CG, CO, EPI>(smem_u32(sA), smem_u32(sB), tmem);
-    umma::commit(bar);
-  }
-  __syncwarp();
-  const bool ok = wait_mma(bar, 0, err);
-  umma::fence_after_sync();
-  if (ok) drain_row_tile<CO, EPI>(tmem, warp, lane, kRowThreads / 32, rt, h, w, sbias, zprev, out0, out1);
-  umma::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) {
-    umma::fence_after_sync();
-    umma::tmem_dealloc(tmem, kCols);
-  }
-}
-
-// Persistent, warp-specialised form of the row kernel: one CTA per SM
-// loops over the row tiles; four producer warps stage tile k + 1 (16-byte
-// asynchronous copies) while one thread issues tile k's MMAs and eight
-// warps drain tile k - 1 from tensor memory.  Two staging buffers and two
-// accumulator buffers; the hand-offs are mbarriers:
-//   full[b]   producers -> MMA      staging buffer b holds its tile
-//   empty[b]  MMA commit -> producers  the MMAs that read buffer b are done
-//   tfull[b]  MMA commit -> epilogue   accumulator buffer b is complete
-//   tempty[b] epilogue -> MMA          accumulator buffer b has been read
-// Every wait is bounded; on expiry the CTA records the error and leaves.
-constexpr int kPipeEpiWarps = 8, kPipeProdWarps = 4;
-constexpr int kPipeThreads = 32 * (kPipeEpiWarps + kPipeProdWarps + 1);
-
-template <int CG, int CO>
-struct PipeSmem {
-  using R = RowSmem<CG, CO>;
-  static constexpr uint32_t kStage = (R::kBytesA + 127u) & ~127u;  // one staging buffer (A operand)
-  static constexpr uint32_t kOffB = 2u * kStage;
-  static constexpr uint32_t kOffBar = (kOffB + R::kBytesB + 7u) & ~7u;
-  static constexpr uint32_t kBytes = kOffBar + 8u * 8u + 16u;
-  static constexpr uint32_t kColsBuf = umma::tmem_cols(kRows * CO);
-  static constexpr uint32_t kTmemCols = 2u * kColsBuf;
-  // At most 512 / kTmemCols CTAs per SM (see RowSmem).
-  static constexpr uint32_t kMaxCtas = 512u / kTmemCols;
-  static constexpr uint32_t kMinBytes = (228u * 1024u) / (kMaxCtas + 1u) + 1024u;
-  static constexpr uint32_t kLaunchBytes = kBytes > kMinBytes ? kBytes : kMinBytes;
-};
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -462,17 +255,59 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, kWaitPolls));
 }
 
+// Forward / backward-data kernel, any image size: persistent CTAs, one per SM,
+// loop over row tiles.  A tile is 8 image rows x 128 pixels; its 10 x 130 input
+// pixels (periodic) are staged once as NHWC has them (umma.cuh: a swizzled K-major
+// M = 128 operand whose rows are pixels), so the nine taps need no copies
+// (issue_row_mmas).  Five producer warps stage tile k + 1
+// while one thread issues tile k's MMAs and sixteen warps drain tile k - 1 from
+// tensor memory (128 lanes x CO columns per row, eight rows side by side); two
+// staging and two accumulator buffers, hand-offs by mbarriers:
+//   full[b]   producers -> MMA      staging buffer b holds its tile
+//   empty[b]  MMA commit -> producers  the MMAs that read buffer b are done
+//   tfull[b]  MMA commit -> epilogue   accumulator buffer b is complete
+//   tempty[b] epilogue -> MMA          accumulator buffer b has been read
+// Every wait is bounded; on expiry the CTA records the error and leaves.
+// One 32 -> 32 GELU layer over 8 x 512^2 moves 403 MB (62 us at the 6.45 TB/s copy
+// rate): 111 us a call, about 75 of them the kernel's, against 174 before the
+// swizzled staging (full L2 sectors: 131 -> 114), the N = 3 CO MMAs, constant
+// descriptor steps and sixteen epilogue warps with 32-byte stores.  What is left
+// over the copy: the 16 special-function operations a clock of GELU (2.2 us of a
+// tile's 4.4), the first tile's load and the last one's drain.
+constexpr int kPipeEpiWarps = 16, kPipeProdWarps = 5;
+constexpr int kPipeThreads = 32 * (kPipeEpiWarps + kPipeProdWarps + 1);
+
+template <int CG, int CO>
+struct PipeSmem {
+  static constexpr uint32_t kStage = ((kRows + 2) * kRowPitch * 2u * CG + 1023u) & ~1023u;  // one staging buffer
+  static constexpr uint32_t kOffB = 2u * kStage;
+  static constexpr uint32_t kBytesB = (uint32_t)CO * 9u * CG * 2u;
+  static constexpr uint32_t kOffBar = (kOffB + kBytesB + 7u) & ~7u;
+  static constexpr uint32_t kBytes = kOffBar + 8u * 8u + 16u;
+  static constexpr uint32_t kColsBuf = umma::tmem_cols(kRows * CO);
+  static constexpr uint32_t kTmemCols = 2u * kColsBuf;
+  // Shared memory requested per CTA: at least enough that no more CTAs fit
+  // on an SM (228 KB) than its 512 tensor-memory columns hold.
+  static constexpr uint32_t kMaxCtas = 512u / kTmemCols;
+  static constexpr uint32_t kMinBytes = (228u * 1024u) / (kMaxCtas + 1u) + 1024u;
+  static constexpr uint32_t kLaunchBytes = kBytes > kMinBytes ? kBytes : kMinBytes;
+};
+
+// EPI: CONV_GELU   out0 = z (bf16), out1 = gelu(z) (bf16), z = acc + bias
+//      CONV_LINEAR out0 = acc + bias (fp32)
+//      CONV_DGELU  out0 = acc * gelu'(zprev) (bf16); taps mirrored (the
+//                  transposed convolution of the backward pass)
 template <int CG, int CO, int EPI>
 __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __nv_bfloat16* __restrict__ x,
                                                                        const __nv_bfloat16* __restrict__ wt,
                                                                        const float* __restrict__ bias,
                                                                        const __nv_bfloat16* __restrict__ zprev,
-                                                                       int batch, int h, int w,
+                                                                       long long ntiles, int h, int w,
                                                                        void* __restrict__ out0,
-                                                                       void* __restrict__ out1,
+                                                                       void* __restrict__ out1, int wide,
                                                                        int* __restrict__ err) {
   using S = PipeSmem<CG, CO>;
-  extern __shared__ __align__(128) unsigned char smem[];
+  extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* sB = smem + S::kOffB;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
   uint64_t* empty = full + 2;
@@ -481,7 +316,6 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
   uint32_t* tslot = reinterpret_cast<uint32_t*>(full + 8);
   __shared__ __align__(16) float sbias[CO];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long long ntiles = (long long)batch * (h / kRows) * (w / kRowPix);
 
   if (warp == 0) {
     umma::tmem_alloc(tslot, S::kTmemCols);
@@ -492,12 +326,12 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
       mbar_init(full + b, kPipeProdWarps * 32);
       mbar_init(empty + b, 1);
       mbar_init(tfull + b, 1);
-      mbar_init(tempty + b, kPipeEpiWarps * 32);
+      mbar_init(tempty + b, kPipeEpiWarps);
     }
     fence_barrier_init();
   }
   if (tid < CO) sbias[tid] = EPI == CONV_DGELU ? 0.0f : bias[tid];
-  stage_weights<CG, CO>(sB, wt, tid, kPipeThreads);
+  stage_weights<CG, CO, EPI>(sB, wt, tid, kPipeThreads);
   fence_proxy_async_smem();
   umma::fence_before_sync();
   __syncthreads();
@@ -508,7 +342,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
   if (warp >= kPipeEpiWarps && warp < kPipeEpiWarps + kPipeProdWarps) {
     // Producers: stage tile k into buffer k % 2 once the MMAs of tile k - 2
     // (the buffer's previous tile) are done.
-    const int pt = tid - kPipeEpiWarps * 32;
+    const int pw = warp - kPipeEpiWarps;
     int k = 0;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
       const int b = k & 1;
@@ -516,8 +350,11 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
         ok = false;
         break;
       }
-      stage_row_tile<CG>(smem + b * S::kStage, x, row_tile(tile, h, w), h, w, pt, kPipeProdWarps * 32);
-      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      const RowTile rt = row_tile<kRows, kRowPix>(tile, h, w);
+      const uint32_t dst = smem_u32(smem + b * S::kStage);
+      for (int r = pw; r < kRows + 2; r += kPipeProdWarps)
+        stage_halo_row<CG, kRowPix, false>(dst + r * kRowPitch * 2 * CG, x, rt, r, h, w, lane);
+      cp_wait_all();
       fence_proxy_async_smem();
       mbar_arrive(full + b);
     }
@@ -534,8 +371,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
       }
       umma::fence_after_sync();
       if (lane == 0) {
-        issue_row_mmas<CG, CO, EPI>(smem_u32(smem + b * S::kStage), smem_u32(sB),
-                                    tmem + (uint32_t)b * S::kColsBuf);
+        issue_row_mmas<CG, CO>(smem_u32(smem + b * S::kStage), smem_u32(sB), tmem + (uint32_t)b * S::kColsBuf,
+                                    row_tile<kRows, kRowPix>(tile, h, w).rows);
         umma::commit(tfull + b);
         umma::commit(empty + b);
       }
@@ -546,7 +383,9 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
     for (int kk = k - 2; ok && kk < k; kk++)
       if (kk >= 0 && !warp_wait(empty + (kk & 1), (uint32_t)(kk >> 1) & 1u)) ok = false;
   } else {
-    // Epilogue warps: tile k from accumulator buffer k % 2.
+    // Epilogue warps: tile k from accumulator buffer k % 2; warp q + 4 r owns
+    // lane quarter q (pixels 32 q .. 32 q + 31) of rows r and r + 4.
+    const int q = warp & 3;
     int k = 0;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
       const int b = k & 1;
@@ -555,10 +394,24 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
         break;
       }
       umma::fence_after_sync();
-      drain_row_tile<CO, EPI>(tmem + (uint32_t)b * S::kColsBuf, warp, lane, kPipeEpiWarps, row_tile(tile, h, w), h,
-                              w, sbias, zprev, out0, out1);
+      const RowTile rt = row_tile<kRows, kRowPix>(tile, h, w);
+      if (q * 32 < rt.pix) {
+        const bool in = q * 32 + lane < rt.pix;
+#pragma unroll 1
+        for (int r = warp >> 2; r < rt.rows; r += kPipeEpiWarps / 4) {
+          const long long p = (rt.bb * h + rt.y0 + r) * (long long)w + rt.x0 + q * 32 + lane;
+          const uint32_t t0 = tmem + (uint32_t)b * S::kColsBuf + ((uint32_t)(q * 32) << 16) + (uint32_t)(r * CO);
+#pragma unroll
+          for (int c = 0; c < CO; c += 16) {
+            float acc[16];
+            umma::ld16(t0 + c, acc);
+            if (in) epilogue16<CO, EPI>(acc, c, p, sbias, zprev, out0, out1, wide != 0);
+          }
+        }
+      }
       umma::fence_before_sync();
-      mbar_arrive(tempty + b);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty + b);
     }
   }
   if (!ok && lane == 0) atomicExch(err, PMHD_LEARNED_ERR_TIMEOUT);
@@ -570,157 +423,204 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
   }
 }
 
-template <int CIN, int CO>
+// Weight gradient, any image size.  K = pixels, so both operands are MN-major
+// with NHWC's channels along M and N, staged as NHWC has them (umma.cuh).  Staged
+// rows are equidistant, so rows 2 q .. 2 q + 3 of x are four channel blocks of an
+// M = 128 operand, and output rows 2 q, 2 q + 1 of dz the two of an N = 2 CO one.
+// For each dx (a shift of x's start address by a pixel)
+// D_dx[(row i, c_in)][(row o, c_out)] accumulates over all tiles of the CTA; the
+// blocks with i - 1 - o in {-1, 0, 1} are the three vertical taps (six of eight
+// blocks useful).  48 MMAs of N = 64 a tile of 8 x 64 pixels.  Six producer warps
+// fill three stages; four warps sum dz for the bias gradient from the staged
+// tiles (when asked to) and add the CTA's accumulators to dw at the end.
+// 32 -> 32 over 8 x 512^2 reads 268 MB (42 us at the copy rate): about 70 us
+// against 1,110 for transposing 8 x 8 blocks of nine gathered copies into K-major
+// tiles, 64 pixels at a time without overlap; 90 without swizzle (16-byte
+// planes fetch every 32-byte sector twice).
+constexpr int kWgRows = 8, kWgPix = 64, kWgStages = 3;
+constexpr int kWgEpiWarps = 4, kWgProdWarps = 6;
+constexpr int kWgThreads = 32 * (kWgEpiWarps + kWgProdWarps + 1);
+
+template <int CO>
 struct WgradSmem {
-  static constexpr int M = 9 * CIN;
-  static constexpr int MT = (M + 127) / 128;           // M = 128 tiles
-  static constexpr int KC = 64;                        // pixels per chunk
-  static constexpr uint32_t kLboA = MT * 16u * 128u;   // K-group (8 pixels) stride of A
-  static constexpr uint32_t kBytesA = (KC / 8) * kLboA;
-  static constexpr uint32_t kLboB = (CO / 8) * 128u;
-  static constexpr uint32_t kBytesB = (KC / 8) * kLboB;
-  static constexpr uint32_t kOffBar = kBytesA + kBytesB;
-  static constexpr uint32_t kBytes = kOffBar + 16u;
+  static constexpr uint32_t kXRow = (kWgPix + 2) * 64u;  // row stride of x
+  static constexpr uint32_t kBytesX = ((kWgRows + 2) * kXRow + 1023u) & ~1023u;
+  static constexpr uint32_t kDRow = kWgPix * 2u * CO;    // row stride of dz
+  static constexpr uint32_t kBytesD = kWgRows * kDRow;
+  static constexpr uint32_t kStage = kBytesX + kBytesD;
+  static constexpr uint32_t kOffBar = kWgStages * kStage;
+  static constexpr uint32_t kBytes = kOffBar + (2u * kWgStages + 1u) * 8u + 8u;
+  static constexpr uint32_t kTmemCols = umma::tmem_cols(3 * 2 * CO);
+  static_assert(kStage % 1024 == 0, "the bias sums take a stage's base out of the swizzle");
+  static_assert(2 * kBytes > 228 * 1024, "one CTA per SM (tensor memory)");
 };
 
-// dW[co][t][ci] += sum_p dz[p][co] * x[p + tap t][ci] over this CTA's pixel
-// chunks; accumulator tile i (rows m = 128 i + lane, m = t * CIN + ci) sits
-// in tensor-memory columns [32 i, 32 i + CO).
-template <int CIN, int CO>
-__global__ void __launch_bounds__(128) wgrad_kernel(const __nv_bfloat16* __restrict__ x,
-                                                    const __nv_bfloat16* __restrict__ dz, int batch, int h, int w,
-                                                    float* __restrict__ dw, int* __restrict__ err) {
-  using S = WgradSmem<CIN, CO>;
-  constexpr uint32_t kCols = umma::tmem_cols(32 * S::MT);
-  extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char* sA = smem;
-  unsigned char* sB = smem + S::kBytesA;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::kOffBar + 8);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const long long P = (long long)batch * h * w;
-  const long long nchunks = (P + S::KC - 1) / S::KC;
+template <int CO>
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __nv_bfloat16* __restrict__ x,
+                                                              const __nv_bfloat16* __restrict__ dz, long long ntiles,
+                                                              int h, int w, float* __restrict__ dw,
+                                                              float* __restrict__ db, int* __restrict__ err) {
+  using S = WgradSmem<CO>;
+  constexpr int NG = CO / 8;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
+  uint64_t* empty = full + kWgStages;
+  uint64_t* done = empty + kWgStages;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
-    umma::tmem_alloc(tslot, kCols);
+    umma::tmem_alloc(tslot, S::kTmemCols);
     umma::tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(bar, 1);
+    for (int b = 0; b < kWgStages; b++) {
+      mbar_init(full + b, kWgProdWarps * 32);
+      mbar_init(empty + b, db ? 1 + kWgEpiWarps : 1);
+    }
+    mbar_init(done, 1);
     fence_barrier_init();
-  }
-  // Rows M .. 128*MT-1 of A stay zero.
-  constexpr int kPadGroups = S::MT * 16 - S::M / 8;
-  for (int c = tid; c < (S::KC / 8) * kPadGroups * 8; c += 128) {
-    const int kg = c / (kPadGroups * 8), r = c - kg * kPadGroups * 8;
-    *reinterpret_cast<uint4*>(sA + kg * S::kLboA + (S::M / 8) * 128 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
   }
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = *tslot;
-  constexpr uint32_t idesc = umma::idesc_bf16(128, CO, false, false);
-  const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-  uint32_t phase = 0;
-  bool ok = true, any = false;
-  for (long long ch = blockIdx.x; ch < nchunks && ok; ch += gridDim.x) {
-    const long long p0 = ch * S::KC;
-    // A: blocks of 8 pixels x 8 channels, transposed in registers so that
-    // each row (one tap and channel) holds 8 consecutive pixels (K-major).
-    for (int c = tid; c < 9 * (S::KC / 8) * (CIN / 8); c += 128) {
-      const int g = c % (CIN / 8);
-      const int kg = (c / (CIN / 8)) % (S::KC / 8);
-      const int t = c / ((S::KC / 8) * (CIN / 8));
-      uint4 v[8];
+  bool ok = true;
+
+  if (warp >= kWgEpiWarps && warp < kWgEpiWarps + kWgProdWarps) {
+    // Producers: ten input rows and eight gradient rows a tile, three a warp.
+    const int pw = warp - kWgEpiWarps;
+    int k = 0;
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
+      const int b = k % kWgStages;
+      if (k >= kWgStages && !warp_wait(empty + b, (uint32_t)(k / kWgStages - 1) & 1u)) {
+        ok = false;
+        break;
+      }
+      const RowTile rt = row_tile<kWgRows, kWgPix>(tile, h, w);
+      const uint32_t dst = smem_u32(smem + b * S::kStage);
+      for (int r = pw; r < 2 * kWgRows + 2; r += kWgProdWarps) {
+        if (r < kWgRows + 2) {
+          stage_halo_row<32, kWgPix, true>(dst + r * S::kXRow, x, rt, r, h, w, lane);
+        } else {
+          const int o = r - (kWgRows + 2);
+          const bool row_in = o < rt.rows;
+          const __nv_bfloat16* src =
+              dz + ((rt.bb * h + rt.y0 + (row_in ? o : 0)) * (long long)w + rt.x0) * CO + lane % NG * 8;
+          const uint32_t d = umma::swz<2 * CO>(dst + S::kBytesX + o * S::kDRow + lane * 16);
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        v[q] = make_uint4(0u, 0u, 0u, 0u);
-        const long long p = p0 + kg * 8 + q;
-        if (p < P) {
-          const int x0 = (int)(p % w);
-          const long long r = p / w;
-          const int y0 = (int)(r % h);
-          const long long b = r / h;
-          const int yy = wrap(y0 + t / 3 - 1, h), xx = wrap(x0 + t % 3 - 1, w);
-          v[q] = *reinterpret_cast<const uint4*>(x + ((b * h + yy) * (long long)w + xx) * CIN + g * 8);
+          for (int i = 0; i < kWgPix * NG / 32; i++) {
+            const int px = lane / NG + i * (32 / NG);
+            const bool take = row_in && px < rt.pix;
+            cp16_or_zero(d + i * 512, src + (take ? px * CO : 0), take);
+          }
         }
       }
-#pragma unroll
-      for (int ch = 0; ch < 8; ch++) {
-        const int m = t * CIN + g * 8 + ch;
-        *reinterpret_cast<uint4*>(sA + (m / 8) * 128 + (m % 8) * 16 + kg * S::kLboA) = transpose_row(v, ch);
+      cp_wait_all();
+      fence_proxy_async_smem();
+      mbar_arrive(full + b);
+    }
+  } else if (warp == kWgEpiWarps + kWgProdWarps) {
+    constexpr uint32_t idesc = umma::idesc_bf16(128, 2 * CO, true, true);
+    int k = 0;
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
+      const int b = k % kWgStages;
+      if (!warp_wait(full + b, (uint32_t)(k / kWgStages) & 1u)) {
+        ok = false;
+        break;
       }
-    }
-    // B: the output gradient, the same way (rows = output channels).
-    for (int c = tid; c < (S::KC / 8) * (CO / 8); c += 128) {
-      const int g = c % (CO / 8), kg = c / (CO / 8);
-      uint4 v[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const long long p = p0 + kg * 8 + q;
-        v[q] = p < P ? *reinterpret_cast<const uint4*>(dz + p * CO + g * 8) : make_uint4(0u, 0u, 0u, 0u);
-      }
-#pragma unroll
-      for (int ch = 0; ch < 8; ch++)
-        *reinterpret_cast<uint4*>(sB + g * 128 + ch * 16 + kg * S::kLboB) = transpose_row(v, ch);
-    }
-    fence_proxy_async_smem();
-    umma::fence_before_sync();
-    __syncthreads();
-    umma::fence_after_sync();
-    if (tid == 0) {
-#pragma unroll
-      for (int kk = 0; kk < S::KC / 16; kk++)
-#pragma unroll
-        for (int i = 0; i < S::MT; i++) {
-          const uint64_t da = umma::desc(a0 + i * 2048 + kk * 2 * S::kLboA, S::kLboA, 128);
-          const uint64_t db = umma::desc(b0 + kk * 2 * S::kLboB, S::kLboB, 128);
-          umma::mma_bf16(tmem + 32 * i, da, db, idesc, (any || kk) ? 1u : 0u);
-        }
-      umma::commit(bar);
-    }
-    __syncwarp();
-    ok = wait_mma(bar, phase, err);
-    phase ^= 1u;
-    any = true;
-    umma::fence_after_sync();
-    ok = __syncthreads_and(ok);  // every warp agrees before the tiles are rewritten
-  }
-  if (any && ok) {
+      umma::fence_after_sync();
+      if (lane == 0) {
+        const uint32_t a0 = smem_u32(smem + b * S::kStage);
+        const uint64_t da = umma::desc(a0, S::kXRow, 512, umma::kSwizzle64);
+        const uint64_t dd =
+            umma::desc(a0 + S::kBytesX, S::kDRow, 16 * CO, CO == 32 ? umma::kSwizzle64 : umma::kSwizzle32);
+        const uint32_t a_hi = umma::desc_hi(da), d_hi = umma::desc_hi(dd);
+        uint32_t a_lo = umma::desc_lo(da), d_lo = umma::desc_lo(dd);
+        const int pairs = (row_tile<kWgRows, kWgPix>(tile, h, w).rows + 1) / 2;
 #pragma unroll 1
-    for (int i = 0; i < S::MT; i++) {
-      float acc[CO];
+        for (int q = 0; q < pairs; q++, a_lo += 2 * S::kXRow / 16, d_lo += 2 * S::kDRow / 16)
 #pragma unroll
-      for (int c8 = 0; c8 < CO / 8; c8++)
-        umma::ld8(tmem + ((uint32_t)(warp * 32) << 16) + 32 * i + c8 * 8, acc + c8 * 8);
-      const int m = 128 * i + tid;
-      if (m < S::M)
+          for (int kk = 0; kk < kWgPix; kk += 16)
 #pragma unroll
-        for (int co = 0; co < CO; co++) atomicAdd(dw + (size_t)co * S::M + m, acc[co]);
+            for (int dx = 0; dx < 3; dx++)
+              umma::mma_bf16(tmem + dx * 2 * CO, a_lo + (kk + dx) * 4, a_hi, d_lo + kk * (CO / 8), d_hi, idesc,
+                             (k | q | kk) ? 1u : 0u);
+        umma::commit(empty + b);
+      }
+      __syncwarp();
+    }
+    // Every MMA has completed (also after a failed wait) before the accumulators
+    // are read or released.
+    if (lane == 0) umma::commit(done);
+    __syncwarp();
+    if (!warp_wait(done, 0)) ok = false;
+  } else {
+    if (db) {
+      // Bias gradient: thread (px, half) sums its pixel column's NG / 2 groups.
+      float s[NG / 2][8];
+#pragma unroll
+      for (int g = 0; g < NG / 2; g++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) s[g][c] = 0.f;
+      const int px = tid & 63, half = tid >> 6;
+      int k = 0;
+      for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
+        const int b = k % kWgStages;
+        if (!warp_wait(full + b, (uint32_t)(k / kWgStages) & 1u)) {
+          ok = false;
+          break;
+        }
+        const unsigned char* d = smem + b * S::kStage + S::kBytesX;
+#pragma unroll
+        for (int o = 0; o < kWgRows; o++)
+#pragma unroll
+          for (int g = 0; g < NG / 2; g++) {
+            const uint4 v = *reinterpret_cast<const uint4*>(
+                d + o * S::kDRow + umma::swz<2 * CO>(px * 2 * CO + (half * (NG / 2) + g) * 16));
+            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              s[g][2 * c] += __uint_as_float(u[c] << 16);
+              s[g][2 * c + 1] += __uint_as_float(u[c] & 0xffff0000u);
+            }
+          }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + b);
+      }
+#pragma unroll
+      for (int g = 0; g < NG / 2; g++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+          float v = s[g][c];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == 0 && ok) atomicAdd(db + (half * (NG / 2) + g) * 8 + c, v);
+        }
+    }
+    // Accumulators: lane = (row i = warp, c_in = lane), columns (dx, row o, c_out).
+    if (ok && !warp_wait(done, 0)) ok = false;
+    umma::fence_after_sync();
+    if (ok) {
+#pragma unroll 1
+      for (int c = 0; c < 3 * 2 * CO; c += 16) {
+        float acc[16];
+        umma::ld16(tmem + ((uint32_t)(warp * 32) << 16) + c, acc);
+        const int dx = c / (2 * CO), o = (c / CO) & 1, co = c % CO, dy = warp - 1 - o;
+        if (dy < -1 || dy > 1) continue;
+        float* dst = dw + ((size_t)co * 9 + (dy + 1) * 3 + dx) * 32 + lane;
+#pragma unroll
+        for (int q = 0; q < 16; q++) atomicAdd(dst + (size_t)q * 9 * 32, acc[q]);
+      }
     }
   }
+  if (!ok && lane == 0) atomicExch(err, PMHD_LEARNED_ERR_TIMEOUT);
   umma::fence_before_sync();
   __syncthreads();
   if (warp == 0) {
     umma::fence_after_sync();
-    umma::tmem_dealloc(tmem, kCols);
+    umma::tmem_dealloc(tmem, S::kTmemCols);
   }
-}
-
-// db[co] += sum_p dz[p][co].
-template <int CO>
-__global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16* __restrict__ dz, long long P,
-                                                        float* __restrict__ db) {
-  __shared__ float part[CO];
-  if (threadIdx.x < CO) part[threadIdx.x] = 0.f;
-  __syncthreads();
-  const int c = threadIdx.x % CO;
-  float s = 0.f;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < P * CO; i += (long long)gridDim.x * blockDim.x)
-    s += __bfloat162float(dz[(i / CO) * CO + c]);
-  atomicAdd(&part[c], s);
-  __syncthreads();
-  if (threadIdx.x < CO) atomicAdd(db + threadIdx.x, part[threadIdx.x]);
 }
 
 template <class K>
@@ -730,63 +630,35 @@ cudaError_t set_smem(K kernel, uint32_t bytes) {
 
 int g_sms = 0;  // SM count of the device the kernels were prepared on
 
-// Images whose width is a multiple of 128 and height a multiple of kRows take
-// the row kernels (the tile is staged once; taps are descriptor shifts) --
-// the persistent pipelined one from two row tiles per SM, else one CTA per
-// tile -- others the gather kernel.
+bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
+
+// Persistent CTAs: one per SM, at most one per tile.  Test hook:
+// PMHD_CONV_MAX_CTAS > 0 limits them, so small images still give each CTA several
+// tiles (all buffers reused, barrier phases flipping).
+unsigned persistent_grid(long long tiles) {
+  const int sms = g_sms > 0 ? g_sms : 148;
+  const char* hook_env = getenv("PMHD_CONV_MAX_CTAS");
+  const long long hook = hook_env ? atoll(hook_env) : 0;
+  long long grid = tiles < sms ? tiles : sms;
+  if (hook > 0 && grid > hook) grid = hook;
+  return (unsigned)grid;
+}
+
 template <int CG, int CO, int EPI>
 cudaError_t launch_conv(const __nv_bfloat16* x, int batch, int h, int w, const __nv_bfloat16* wt, const float* bias,
                         const __nv_bfloat16* zprev, void* out0, void* out1, int* err, cudaStream_t s) {
-  if (w % kRowPix == 0 && h % kRows == 0) {
-    const long long tiles = (long long)batch * (h / kRows) * (w / kRowPix);
-    const int sms = g_sms > 0 ? g_sms : 148;
-    // Test hook: PMHD_CONV_MAX_CTAS > 0 selects the persistent kernel on any
-    // row shape with at most that many CTAs, so small images still give each
-    // CTA several tiles (both buffers reused, barrier phases flipping).
-    const char* hook_env = getenv("PMHD_CONV_MAX_CTAS");
-    const long long hook = hook_env ? atoll(hook_env) : 0;
-    if (hook > 0 || tiles >= 2LL * sms) {
-      // Persistent, pipelined: pays off from two tiles per SM (8 x 512^2:
-      // 210 -> 182 us); one tile per CTA gains nothing from the pipeline.
-      long long grid = tiles < sms ? tiles : sms;
-      if (hook > 0 && grid > hook) grid = hook;
-      conv3x3_pipe_kernel<CG, CO, EPI><<<(unsigned)grid, kPipeThreads, PipeSmem<CG, CO>::kLaunchBytes, s>>>(
-          x, wt, bias, zprev, batch, h, w, out0, out1, err);
-      return cudaGetLastError();
-    }
-    const long long ctas = (long long)batch * (h / kRows) * (w / kRowPix);
-    conv3x3_rows_kernel<CG, CO, EPI><<<(unsigned)ctas, kRowThreads, RowSmem<CG, CO>::kLaunchBytes, s>>>(
-        x, wt, bias, zprev, batch, h, w, out0, out1, err);
-    return cudaGetLastError();
-  }
-  using S = ConvSmem<CG, CO>;
-  auto k = conv3x3_kernel<CG, CO, EPI>;
-  const long long P = (long long)batch * h * w;
-  const unsigned grid = (unsigned)((P + 127) / 128);
-  k<<<grid, 128, S::kBytes, s>>>(x, wt, bias, zprev, batch, h, w, out0, out1, err);
+  const long long tiles = (long long)batch * ((h + kRows - 1) / kRows) * ((w + kRowPix - 1) / kRowPix);
+  const int wide = aligned32(out0) && (EPI != CONV_GELU || aligned32(out1)) && (EPI != CONV_DGELU || aligned32(zprev));
+  conv3x3_pipe_kernel<CG, CO, EPI><<<persistent_grid(tiles), kPipeThreads, PipeSmem<CG, CO>::kLaunchBytes, s>>>(
+      x, wt, bias, zprev, tiles, h, w, out0, out1, wide, err);
   return cudaGetLastError();
 }
 
-template <int CIN, int CO>
+template <int CO>
 cudaError_t launch_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dz, int batch, int h, int w, float* dw,
                          float* db, int* err, cudaStream_t s) {
-  using S = WgradSmem<CIN, CO>;
-  auto k = wgrad_kernel<CIN, CO>;
-  const int sms = g_sms > 0 ? g_sms : 148;
-  const long long P = (long long)batch * h * w;
-  const long long nchunks = (P + S::KC - 1) / S::KC;
-  // Up to 4 CTAs per SM fit both shared memory and the 512 tensor-memory
-  // columns; each CTA takes several chunks so the atomics stay few.
-  long long grid = nchunks < 2LL * sms ? nchunks : 2LL * sms;
-  if (grid < 1) grid = 1;
-  k<<<(unsigned)grid, 128, S::kBytes, s>>>(x, dz, batch, h, w, dw, err);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || !db) return e;
-  const long long tot = P * CO;
-  long long bg = (tot + 255) / 256;
-  if (bg > 4LL * sms) bg = 4LL * sms;
-  if (bg < 1) bg = 1;
-  bias_grad_kernel<CO><<<(unsigned)bg, 256, 0, s>>>(dz, P, db);
+  const long long tiles = (long long)batch * ((h + kWgRows - 1) / kWgRows) * ((w + kWgPix - 1) / kWgPix);
+  wgrad_kernel<CO><<<persistent_grid(tiles), kWgThreads, WgradSmem<CO>::kBytes, s>>>(x, dz, tiles, h, w, dw, db, err);
   return cudaGetLastError();
 }
 
@@ -796,20 +668,12 @@ cudaError_t conv_prepare() {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = set_smem(conv3x3_kernel<32, 32, CONV_GELU>, ConvSmem<32, 32>::kBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_kernel<32, 16, CONV_LINEAR>, ConvSmem<32, 16>::kBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_kernel<16, 32, CONV_DGELU>, ConvSmem<16, 32>::kBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_kernel<32, 32, CONV_DGELU>, ConvSmem<32, 32>::kBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_rows_kernel<32, 32, CONV_GELU>, RowSmem<32, 32>::kLaunchBytes);
   if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<32, 32, CONV_GELU>, PipeSmem<32, 32>::kLaunchBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_rows_kernel<32, 16, CONV_LINEAR>, RowSmem<32, 16>::kLaunchBytes);
   if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<32, 16, CONV_LINEAR>, PipeSmem<32, 16>::kLaunchBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_rows_kernel<16, 32, CONV_DGELU>, RowSmem<16, 32>::kLaunchBytes);
   if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<16, 32, CONV_DGELU>, PipeSmem<16, 32>::kLaunchBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_rows_kernel<32, 32, CONV_DGELU>, RowSmem<32, 32>::kLaunchBytes);
   if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<32, 32, CONV_DGELU>, PipeSmem<32, 32>::kLaunchBytes);
-  if (e == cudaSuccess) e = set_smem(wgrad_kernel<32, 32>, WgradSmem<32, 32>::kBytes);
-  if (e == cudaSuccess) e = set_smem(wgrad_kernel<32, 16>, WgradSmem<32, 16>::kBytes);
+  if (e == cudaSuccess) e = set_smem(wgrad_kernel<32>, WgradSmem<32>::kBytes);
+  if (e == cudaSuccess) e = set_smem(wgrad_kernel<16>, WgradSmem<16>::kBytes);
   return e;
 }
 
@@ -829,8 +693,8 @@ cudaError_t conv3x3(int mode, const __nv_bfloat16* x, int batch, int h, int w, i
 
 cudaError_t conv3x3_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dz, int batch, int h, int w, int c_in,
                           int c_out, float* dw, float* db, int* err, cudaStream_t s) {
-  if (c_in == 32 && c_out == 32) return launch_wgrad<32, 32>(x, dz, batch, h, w, dw, db, err, s);
-  if (c_in == 32 && c_out == 16) return launch_wgrad<32, 16>(x, dz, batch, h, w, dw, db, err, s);
+  if (c_in == 32 && c_out == 32) return launch_wgrad<32>(x, dz, batch, h, w, dw, db, err, s);
+  if (c_in == 32 && c_out == 16) return launch_wgrad<16>(x, dz, batch, h, w, dw, db, err, s);
   return cudaErrorNotSupported;
 }
 

@@ -3,13 +3,18 @@
 // the BF16 instruction descriptor, tcgen05.mma / commit, tensor-memory
 // allocation and tcgen05.ld, written as inline PTX.
 //
-// Operand layouts are the "no swizzle" canonical layouts of the tcgen05
-// matrix descriptors, in bytes (bf16 elements, a core matrix is 8 rows of
-// 16 bytes):
-//   K-major  (row r of M or N, k along K): (r%8)*16 + (r/8)*SBO + (k%8)*2 + (k/8)*LBO
-//   MN-major (mn along M or N, k along K): (mn%8)*2 + (mn/8)*SBO + (k%8)*16 + (k/8)*LBO
-// With SBO = 128 the rows of a K-major operand sit 16 bytes apart, so a
-// shift by whole rows is a shift of the descriptor's start address.
+// Operand layouts are the canonical layouts of the tcgen05 matrix descriptors
+// (bf16 elements), in bytes.  Weights: K-major without swizzle, core matrices of
+// 8 rows of 16 bytes,
+//   (row r of M or N, k along K): (r%8)*16 + (r/8)*SBO + (k%8)*2 + (k/8)*LBO
+// Images: pixel rows as NHWC has them, 64 bytes (32 channels) or 32 bytes (16),
+// with the 64- or 32-byte swizzle, which exchanges the 16-byte chunks of a pixel
+// by address bits 7-8 (swz below) so that eight pixels' chunks meet all banks:
+//   K-major, pixels along M:       pixel p at (p%8)*B + (p/8)*SBO, k contiguous
+//   MN-major, channels along M/N:  pixel k at (k%8)*B + (k/8)*SBO, channel blocks
+//                                  of B bytes at LBO
+// With SBO = 8 B pixels are equidistant, and as the swizzle goes by address a
+// shift by whole pixels is a shift of the descriptor's start address.
 #ifndef PMHD_LEARNED_UMMA_CUH
 #define PMHD_LEARNED_UMMA_CUH
 
@@ -20,13 +25,22 @@
 namespace pmhd {
 namespace umma {
 
+// Byte address of a 16-byte chunk under the 64-byte (PXB = 64) or 32-byte (32)
+// swizzle.
+template <int PXB>
+__device__ __forceinline__ uint32_t swz(uint32_t addr) {
+  static_assert(PXB == 64 || PXB == 32, "pixel rows of 64 or 32 bytes");
+  return addr ^ ((addr >> 3) & (PXB == 64 ? 0x30u : 0x10u));
+}
+// Descriptor layout types.
+constexpr uint32_t kNoSwizzle = 0, kSwizzle64 = 4, kSwizzle32 = 6;
+
 // Shared-memory matrix descriptor: start address, leading-dimension byte
-// offset (K-group stride), stride-dimension byte offset (8-row-group
-// stride), all >> 4; bits 46-47 = 1 (descriptor version of sm_100);
-// layout type 0 (no swizzle); base offset 0.
-__device__ __forceinline__ uint64_t desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+// offset, stride-dimension byte offset, all >> 4; bits 46-47 = 1 (descriptor
+// version of sm_100); base offset 0; layout type at bits 61-63.
+__device__ __forceinline__ uint64_t desc(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
   return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | ((uint64_t)layout << 61);
 }
 
 // Instruction descriptor of kind::f16 with BF16 A and B, FP32 accumulator:
@@ -38,13 +52,23 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, bool a_mn, bool 
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// D[tmem] (+)= A * B^T, issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+// A descriptor's two words: the address moves the low word by one per 16 bytes
+// (operands below 256 KB of shared memory never carry out of its 14 bits), so
+// the issuing thread keeps one base per operand and adds constants (building
+// each descriptor in 64 bits per MMA: 232 -> 188 us a call of the 8 x 512^2 layer).
+__device__ __forceinline__ uint32_t desc_lo(uint64_t d) { return (uint32_t)d; }
+__device__ __forceinline__ uint32_t desc_hi(uint64_t d) { return (uint32_t)(d >> 32); }
+
+// D[tmem] (+)= A * B^T, issued by one thread; operands by descriptor words.
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                         uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %2};\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -69,25 +93,21 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Eight consecutive 32-bit accumulator columns of this thread's lane (warp
-// w of the CTA reads lanes 32w .. 32w+31), waiting for the load in the same
+// Sixteen consecutive 32-bit accumulator columns of this thread's lane (warp
+// w of the CTA reads lanes 32 (w % 4) .. + 31), waiting for the load in the same
 // statement so the values are never used early.
-__device__ __forceinline__ void ld8(uint32_t taddr, float* v) {
-  uint32_t r0, r1, r2, r3, r4, r5, r6, r7;
+__device__ __forceinline__ void ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];\n\t"
       "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3), "=r"(r4), "=r"(r5), "=r"(r6), "=r"(r7)
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
-  v[0] = __uint_as_float(r0);
-  v[1] = __uint_as_float(r1);
-  v[2] = __uint_as_float(r2);
-  v[3] = __uint_as_float(r3);
-  v[4] = __uint_as_float(r4);
-  v[5] = __uint_as_float(r5);
-  v[6] = __uint_as_float(r6);
-  v[7] = __uint_as_float(r7);
+#pragma unroll
+  for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
 }
 
 // Tensor-memory columns to allocate for `n` accumulator columns (a power of
