@@ -13,6 +13,8 @@
 
 #include <cmath>
 
+#include "pmhd/fastmath.hpp"
+
 #ifndef __CUDACC__
 #ifndef __host__
 #define __host__
@@ -302,8 +304,7 @@ __host__ __device__ inline void hll_flux_1d(const T WL[3], const T WR[3], T f[3]
 //   * every expression in the run's type T (the reference evaluates the gamma
 //     expressions of its binary32 build in binary64);
 //   * one reciprocal per density or divisor, shared by its quotients, and
-//     1 / (gamma - 1) as the constant 2.5 (binary64: the IEEE reciprocal;
-//     binary32: the hardware's approximate reciprocal and square root);
+//     1 / (gamma - 1) as the constant 2.5 (reciprocals and roots: fastmath.hpp);
 //   * the two Hancock faces of a cell share one flux difference (it depends
 //     only on the two face states, riemann.hpp:60-88 forms it twice);
 //   * the HLLC star energy as coeff (E/rho + (S* - u) S*) + (S* - u) p / (S - S*),
@@ -312,18 +313,10 @@ __host__ __device__ inline void hll_flux_1d(const T WL[3], const T WR[3], T f[3]
 #if defined(__CUDACC__)
 namespace fastform {
 
-__device__ __forceinline__ double rcp(double x) { return __drcp_rn(x); }
-__device__ __forceinline__ float rcp(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ double root(double x) { return sqrt(x); }
-__device__ __forceinline__ float root(float x) {
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
+__device__ __forceinline__ double rcp(double x) { return fast_rcp(x); }
+__device__ __forceinline__ float rcp(float x) { return fast_rcp(x); }
+__device__ __forceinline__ double root(double x) { return fast_sqrt(x); }
+__device__ __forceinline__ float root(float x) { return fast_sqrt(x); }
 
 template <class T>
 __device__ __forceinline__ void cons_to_prim(const T U[4], T W[4]) {

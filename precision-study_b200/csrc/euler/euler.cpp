@@ -173,19 +173,6 @@ int build_graph(pmhd_euler2d* e, int nsteps, cudaGraphExec_t* out) {
   return e3 == cudaSuccess ? PMHD_OK : PMHD_ERR_CUDA;
 }
 
-template <class T>
-void prims_from_cons(const std::vector<unsigned char>& buf, const pmhd_euler2d* e, void* host) {
-  const T* u = reinterpret_cast<const T*>(buf.data());
-  T* out = static_cast<T*>(host);
-  for (int j = 0; j < e->ny; j++)
-    for (int i = 0; i < e->nx; i++) {
-      T U[4], W[4];
-      for (int k = 0; k < 4; k++) U[k] = u[(size_t)k * e->plane + (size_t)j * e->pitch + i];
-      cons_to_prim(U, W);
-      for (int k = 0; k < 4; k++) out[((size_t)j * e->nx + i) * 4 + k] = W[k];
-    }
-}
-
 // Toro test states rhoL uL pL rhoR uR pR T_end x0 (riemann1d_cpu.cpp:43-62).
 bool toro(int id, double s[8]) {
   static const double tc[5][8] = {{1.0, 0.0, 1.0, 0.125, 0.0, 0.1, 0.25, 0.5},
@@ -401,14 +388,12 @@ int pmhd_euler2d_advance(pmhd_euler2d* e, double t_end, long long max_steps, pmh
 int pmhd_euler2d_get_prim(pmhd_euler2d* e, void* host) {
   if (!e || !host) return PMHD_ERR_ARG;
   E_CU(cudaSetDevice(e->device));
-  std::vector<unsigned char> buf((size_t)4 * e->plane * e->elem);
-  // Graphs hold an even number of steps, so the state is always in u[0].
-  E_CU(cudaMemcpyAsync(buf.data(), e->u[0], buf.size(), cudaMemcpyDeviceToHost, e->stream));
+  // Graphs hold an even number of steps, so the state is always in u[0] and
+  // u[1] is free between advances: the primitives are formed there (by the
+  // parity build's kernel, whatever the run's flavour) and copied out once.
+  E_CU(exact::prims2d(e->fp32, e->u[0], e->nx, e->ny, e->pitch, e->plane, e->u[1], e->stream));
+  E_CU(cudaMemcpyAsync(host, e->u[1], (size_t)4 * e->nx * e->ny * e->elem, cudaMemcpyDeviceToHost, e->stream));
   E_CU(cudaStreamSynchronize(e->stream));
-  if (e->fp32)
-    prims_from_cons<float>(buf, e, host);
-  else
-    prims_from_cons<double>(buf, e, host);
   return PMHD_OK;
 }
 

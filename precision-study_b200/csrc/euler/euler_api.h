@@ -29,6 +29,8 @@ struct EulerCtrl {
                      double dx, double dy, double cfl, EulerCtrl* ctrl, int p, cudaStream_t s);                     \
   cudaError_t speed2d(int fp32, const void* u, int nx, int ny, int pitch, long long plane, EulerCtrl* ctrl,         \
                       int slot, cudaStream_t s);                                                                    \
+  cudaError_t prims2d(int fp32, const void* u, int nx, int ny, int pitch, long long plane, void* out,               \
+                      cudaStream_t s);                                                                              \
   cudaError_t run1d(int fp32, int hll, void* u, void* f, int n, double t_end, long long max_iters, double* out_t,   \
                     long long* out_steps, int* err, cudaStream_t s);                                                \
   }

@@ -4,18 +4,15 @@
 // one pass over HBM), its initial max-speed reduction, and a one-CTA kernel
 // that runs a whole 1D Riemann problem (src/euler/riemann1d_cpu.cpp:95-196).
 //
-// 2D step kernel.  A CTA of 512 threads owns a 32 x TY tile of output cells
-// (TY = 16 or 12 fp64, 32 fp32).  It loads the conservative state of a
-// (TY + 4) x 36 region around it (2 cells of halo,
-// indices clamped at the walls: the reference's transmissive ghost copies,
-// riemann2d_cpu.cpp:160-182), and runs the first sweep on the part of the
-// region the second sweep needs (all rows for x-then-y, all columns for
-// y-then-x), then the second sweep on the tile; each sweep is
-// reconstruction + Hancock of every cell's two faces, one flux per
-// interface, and the conservative update, staged in shared memory.  The
-// order alternates with the step count (even: x then y).  The next step's
-// max signal speeds come from the epilogue (one atomicMax per CTA), so the
-// time step never needs a separate pass.
+// 2D step kernels.  Indices are clamped at the walls (the reference's transmissive
+// ghost copies, riemann2d_cpu.cpp:160-182); the sweep order alternates with the
+// step count (even: x then y); the next step's max signal speeds come from the
+// epilogue, so the time step never needs a separate pass.  Small binary64 grids:
+// a CTA of 512 threads owns a 32 x 12 tile, loads the 36 x 16 region around it,
+// runs the first sweep on the part of it the second needs, then the second on the
+// tile, each as reconstruction + Hancock of every cell's two faces, one flux per
+// interface and the update, staged in shared memory.  Otherwise: the streaming
+// kernel below.
 //
 // Compiled twice (see Makefile): PMHD_EKNS=exact with -fmad=false (bit
 // parity with the reference CPU build) and PMHD_EKNS=fast (contraction,
@@ -206,8 +203,43 @@ __device__ __forceinline__ void sweep(Tile<T, TY>& s, int r0, int r1, int c0, in
   if (!LAST) __syncthreads();
 }
 
-// Registers: 64 per thread for 1024 / NT resident CTAs (the shared-memory
-// limit of the tile shapes below).
+// The step's control values: every CTA reads the same slots; one thread
+// (advance) writes the other parity and the speed slot two steps ahead.
+template <class T>
+struct StepControl {
+  T t, dt;
+  long long n;
+  bool active;
+  __device__ __forceinline__ StepControl(const EulerCtrl* ctrl, int p, T dx, T dy, T cfl) {
+    t = (T)ctrl->t[p];
+    n = ctrl->step[p];
+    // t and t + dt are values of type T, so their tests against t_end are
+    // exact in binary64 whichever type t_end has.
+    active = !ctrl->stop && (double)t < ctrl->t_end && n < ctrl->step_limit;
+    dt = (T)0;
+    if (active) {
+      const T mx = (T)bits_speed(ctrl->sx[n % 3]), my = (T)bits_speed(ctrl->sy[n % 3]);
+      const T m = vmin(dx / mx, dy / my);
+      dt = ctrl->wide_time ? (T)(ctrl->cfl * (double)m) : cfl * m;
+      if ((double)(T)(t + dt) > ctrl->t_end) dt = ctrl->wide_time ? (T)(ctrl->t_end - (double)t) : (T)ctrl->t_end - t;
+      if (!(dt > (T)0.0) || t + dt == t) active = false;  // riemann2d_cpu.cpp:298, euler2d_cpu.cpp:309
+    }
+  }
+  __device__ __forceinline__ void advance(EulerCtrl* ctrl, int p) const {
+    if (active) {
+      ctrl->t[p ^ 1] = (double)(t + dt);
+      ctrl->step[p ^ 1] = n + 1;
+      ctrl->sx[(n + 2) % 3] = 0ull;
+      ctrl->sy[(n + 2) % 3] = 0ull;
+    } else {
+      ctrl->t[p ^ 1] = ctrl->t[p];
+      ctrl->step[p ^ 1] = n;
+      if ((double)t < ctrl->t_end && n < ctrl->step_limit) ctrl->stop = 1;
+    }
+  }
+};
+
+// Registers: 64 per thread for two resident CTAs of 512.
 template <class T, int TY, int NT, int MINB, bool HLL>
 __global__ void __launch_bounds__(NT, MINB) step_kernel(const T* __restrict__ uin, T* __restrict__ uout, int nx, int ny,
                                                    int pitch, long long plane, T dx, T dy, T cfl, EulerCtrl* ctrl,
@@ -216,31 +248,11 @@ __global__ void __launch_bounds__(NT, MINB) step_kernel(const T* __restrict__ ui
   Tile<T, TY>& s = *reinterpret_cast<Tile<T, TY>*>(smem_raw);
   constexpr int RH = TY + 4;
   const int i0 = blockIdx.x * TW, j0 = blockIdx.y * TY;
-  // Step control (every CTA reads the same slots; block (0,0) writes the
-  // other parity and the speed slot two steps ahead).
-  const T t = (T)ctrl->t[p];
-  const long long n = ctrl->step[p];
-  // t and t + dt are values of type T, so their tests against t_end are
-  // exact in binary64 whichever type t_end has.
-  bool active = !ctrl->stop && (double)t < ctrl->t_end && n < ctrl->step_limit;
-  T dt = (T)0;
-  if (active) {
-    const T mx = (T)bits_speed(ctrl->sx[n % 3]), my = (T)bits_speed(ctrl->sy[n % 3]);
-    const T m = vmin(dx / mx, dy / my);
-    dt = ctrl->wide_time ? (T)(ctrl->cfl * (double)m) : cfl * m;
-    if ((double)(T)(t + dt) > ctrl->t_end) dt = ctrl->wide_time ? (T)(ctrl->t_end - (double)t) : (T)ctrl->t_end - t;
-    if (!(dt > (T)0.0) || t + dt == t) active = false;  // riemann2d_cpu.cpp:298, euler2d_cpu.cpp:309
-  }
-  const bool leader = blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
-  if (!active) {
-    if (leader) {
-      ctrl->t[p ^ 1] = ctrl->t[p];
-      ctrl->step[p ^ 1] = n;
-      if (!((double)t < ctrl->t_end) || n >= ctrl->step_limit) {
-      } else {
-        ctrl->stop = 1;
-      }
-    }
+  const StepControl<T> sc(ctrl, p, dx, dy, cfl);
+  const T dt = sc.dt;
+  const long long n = sc.n;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sc.advance(ctrl, p);
+  if (!sc.active) {
     // Carry the state to the output buffer.
     for (int q = threadIdx.x; q < TW * TY; q += blockDim.x) {
       const int i = i0 + q % TW, j = j0 + q / TW;
@@ -249,12 +261,6 @@ __global__ void __launch_bounds__(NT, MINB) step_kernel(const T* __restrict__ ui
         for (int k = 0; k < NV; k++) uout[k * plane + (long long)j * pitch + i] = uin[k * plane + (long long)j * pitch + i];
     }
     return;
-  }
-  if (leader) {
-    ctrl->t[p ^ 1] = (double)(t + dt);
-    ctrl->step[p ^ 1] = n + 1;
-    ctrl->sx[(n + 2) % 3] = 0ull;
-    ctrl->sy[(n + 2) % 3] = 0ull;
   }
   // Region load with wall clamping, and the primitives of every region cell
   // (same thread, so no barrier between them).  (Measured: asynchronous
@@ -295,6 +301,152 @@ __global__ void __launch_bounds__(NT, MINB) step_kernel(const T* __restrict__ ui
   }
 }
 
+// ---- streaming step kernel -----------------------------------------------------------
+//
+// A warp (a CTA of its own) owns a strip of 28 columns -- its 32 lanes are the
+// strip and two halo columns on each side -- and marches down a block of rows.
+// The sweep along x takes its neighbours by warp shuffles, the sweep along y
+// keeps a window of rows in registers, in either order, so there is no shared
+// memory and no barrier; per output cell 32 / 28 (x) and (rows + 4) / rows of the
+// work is halo.  The next row's loads are issued a row ahead.  Bound by issue and
+// by each warp's dependent chain (a row takes 1.03 us at one warp per scheduler
+// in binary64, 0.57 in binary32).  Registers: 128 / 64 a thread, 16 / 32 warps per
+// SM; one-warp CTAs keep the tile position in uniform registers (four warps a CTA
+// with a position per warp: 124 bytes of spills, 10 % slower).  At 4096^2 fp64
+// 28.3 and fp32 57.8 G zone-cycles/s, against 13.2 / 26.4 with 32 x 16 / 32 x 32
+// shared-memory tiles; at 1024^2 48 / 25 us a step against 89 / 49.
+constexpr int kStripW = 28;
+
+template <class T>
+struct Cell {
+  T v[NV];
+};
+template <class T>
+__device__ __forceinline__ Cell<T> shfl_up1(const Cell<T>& c) {
+  Cell<T> r;
+#pragma unroll
+  for (int k = 0; k < NV; k++) r.v[k] = __shfl_up_sync(0xffffffffu, c.v[k], 1);
+  return r;
+}
+template <class T>
+__device__ __forceinline__ Cell<T> shfl_down1(const Cell<T>& c) {
+  Cell<T> r;
+#pragma unroll
+  for (int k = 0; k < NV; k++) r.v[k] = __shfl_down_sync(0xffffffffu, c.v[k], 1);
+  return r;
+}
+
+// Hancock-evolved lower and upper faces of a cell from its neighbours' and its
+// own primitives along direction NI.
+template <class T, int NI, int TI>
+__device__ __forceinline__ void evolved_faces(const Cell<T>& wm, const Cell<T>& w0, const Cell<T>& wp, T fac,
+                                              Cell<T>& lo, Cell<T>& hi) {
+  T l[NV], r[NV];
+#pragma unroll
+  for (int k = 0; k < NV; k++) muscl_recon(wm.v[k], w0.v[k], wp.v[k], l[k], r[k]);
+  k_hancock_pair<T, NI, TI>(l, r, lo.v, hi.v, fac);
+}
+
+// The x sweep of one row: u is the lane's cell, neighbouring lanes hold its
+// neighbours; valid on lanes 2 .. 29.
+template <class T, bool HLL>
+__device__ __forceinline__ Cell<T> sweep_row_x(const Cell<T>& u, T fac, T ratio) {
+  Cell<T> w, lo, hi, f, r;
+  k_c2p(u.v, w.v);
+  evolved_faces<T, 1, 2>(shfl_up1(w), w, shfl_down1(w), fac, lo, hi);
+  k_flux<T, 1, 2, HLL>(shfl_up1(hi).v, lo.v, f.v);
+  const Cell<T> fr = shfl_down1(f);
+#pragma unroll
+  for (int k = 0; k < NV; k++) r.v[k] = u.v[k] - ratio * (fr.v[k] - f.v[k]);
+  return r;
+}
+
+// The y sweep as a pipeline over rows: push(row r) returns the updated row
+// r - 2 (valid from the fifth push on).
+template <class T, bool HLL>
+struct ColumnSweep {
+  Cell<T> w2, w1, u2, u1, hi2, f2;  // rows r - 2 and r - 1; upper face of row r - 2, flux below it
+  T fac, ratio;
+  __device__ __forceinline__ ColumnSweep(T fac_, T ratio_) : w2{}, w1{}, u2{}, u1{}, hi2{}, f2{}, fac(fac_), ratio(ratio_) {}
+  __device__ __forceinline__ Cell<T> push(const Cell<T>& u) {
+    Cell<T> w, lo, hi, f, r;
+    k_c2p(u.v, w.v);
+    evolved_faces<T, 2, 1>(w2, w1, w, fac, lo, hi);  // faces of row r - 1
+    k_flux<T, 2, 1, HLL>(hi2.v, lo.v, f.v);          // between rows r - 2 and r - 1
+#pragma unroll
+    for (int k = 0; k < NV; k++) r.v[k] = u2.v[k] - ratio * (f.v[k] - f2.v[k]);
+    w2 = w1, w1 = w, u2 = u1, u1 = u, hi2 = hi, f2 = f;
+    return r;
+  }
+};
+
+template <class T, bool HLL, int MINB>
+__global__ void __launch_bounds__(32, MINB) stream_kernel(const T* __restrict__ uin, T* __restrict__ uout, int nx,
+                                                           int ny, int pitch, long long plane, T dx, T dy, T cfl,
+                                                           int rows, EulerCtrl* ctrl, int p) {
+  const StepControl<T> sc(ctrl, p, dx, dy, cfl);
+  const int lane = threadIdx.x, strips = (nx + kStripW - 1) / kStripW;
+  if (blockIdx.x == 0 && lane == 0) sc.advance(ctrl, p);
+  const int strip = (int)(blockIdx.x % (unsigned)strips);
+  const int i = strip * kStripW - 2 + lane, j0 = (int)(blockIdx.x / (unsigned)strips) * rows;
+  const int j1 = j0 + rows < ny ? j0 + rows : ny;
+  const bool owns = lane >= 2 && lane < 2 + kStripW && i < nx;
+  if (!sc.active) {  // carry the state to the output buffer
+    if (owns)
+      for (int j = j0; j < j1; j++)
+#pragma unroll
+        for (int k = 0; k < NV; k++) uout[k * plane + (long long)j * pitch + i] = uin[k * plane + (long long)j * pitch + i];
+    return;
+  }
+  // Indices clamped at the walls: the reference's transmissive ghost copies.
+  const T* col = uin + (i < 0 ? 0 : (i < nx ? i : nx - 1));
+  auto load = [&](int j) {
+    Cell<T> c;
+    const T* q = col + (long long)(j < 0 ? 0 : (j < ny ? j : ny - 1)) * pitch;
+#pragma unroll
+    for (int k = 0; k < NV; k++) c.v[k] = q[k * plane];
+    return c;
+  };
+  unsigned long long bx = 0ull, by = 0ull;
+  auto store = [&](const Cell<T>& c, int j) {
+    if (!owns) return;
+#pragma unroll
+    for (int k = 0; k < NV; k++) uout[k * plane + (long long)j * pitch + i] = c.v[k];
+    T vx, vy;
+    k_speeds(c.v, vx, vy);
+    const unsigned long long sx = speed_bits((double)vx), sy = speed_bits((double)vy);
+    bx = sx > bx ? sx : bx;
+    by = sy > by ? sy : by;
+  };
+  const T dt = sc.dt;
+  const T facx = (T)0.5 * dt / dx, facy = (T)0.5 * dt / dy, rx = dt / dx, ry = dt / dy;
+  ColumnSweep<T, HLL> col_sweep(facy, ry);
+  Cell<T> next = load(j0 - 2);
+  if (sc.n % 2 == 0) {  // x sweep on every row, then y
+#pragma unroll 2
+    for (int j = j0 - 2; j < j1 + 2; j++) {
+      const Cell<T> u = next;
+      next = load(j + 1);
+      const Cell<T> r = col_sweep.push(sweep_row_x<T, HLL>(u, facx, rx));
+      if (j >= j0 + 2) store(r, j - 2);
+    }
+  } else {
+#pragma unroll 2
+    for (int j = j0 - 2; j < j1 + 2; j++) {
+      const Cell<T> u = next;
+      next = load(j + 1);
+      const Cell<T> r = col_sweep.push(u);
+      if (j >= j0 + 2) store(sweep_row_x<T, HLL>(r, facx, rx), j - 2);
+    }
+  }
+  bx = warp_max(bx);
+  by = warp_max(by);
+  if (lane == 0) {
+    if (bx) atomicMax(&ctrl->sx[(sc.n + 1) % 3], bx);
+    if (by) atomicMax(&ctrl->sy[(sc.n + 1) % 3], by);
+  }
+}
+
 template <class T>
 __global__ void __launch_bounds__(256) speed_kernel(const T* __restrict__ u, int nx, int ny, int pitch,
                                                     long long plane, EulerCtrl* ctrl, int slot) {
@@ -315,6 +467,32 @@ __global__ void __launch_bounds__(256) speed_kernel(const T* __restrict__ u, int
   if ((threadIdx.x & 31) == 0) {
     if (bx) atomicMax(&ctrl->sx[slot], bx);
     if (by) atomicMax(&ctrl->sy[slot], by);
+  }
+}
+
+// Primitives [ny][nx][4] of the conservative state, in the reference's
+// expressions (the parity build's flavour gives the bits of the host's
+// cons_to_prim).  Bound by its two passes over memory.
+template <class T>
+__global__ void __launch_bounds__(256) prims_kernel(const T* __restrict__ u, int nx, int ny, int pitch,
+                                                    long long plane, T* __restrict__ out) {
+  for (long long q = blockIdx.x * 256LL + threadIdx.x; q < (long long)nx * ny; q += (long long)gridDim.x * 256) {
+    const int i = (int)(q % nx), j = (int)(q / nx);
+    T U4[NV], W4[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) U4[k] = u[k * plane + (long long)j * pitch + i];
+    cons_to_prim(U4, W4);
+    struct alignas(16) Pair {
+      T a[16 / sizeof(T)];
+    };
+    Pair* o = reinterpret_cast<Pair*>(out + NV * q);
+#pragma unroll
+    for (int k = 0; k < NV; k += (int)(16 / sizeof(T))) {
+      Pair v;
+#pragma unroll
+      for (int m = 0; m < (int)(16 / sizeof(T)); m++) v.a[m] = W4[k + m];
+      o[k / (int)(16 / sizeof(T))] = v;
+    }
   }
 }
 
@@ -411,6 +589,16 @@ cudaError_t launch_step(const void* uin, void* uout, int nx, int ny, int pitch, 
   return cudaGetLastError();
 }
 
+template <class T, int MINB>
+cudaError_t launch_stream(int hll, int rows, const void* uin, void* uout, int nx, int ny, int pitch, long long plane,
+                          double dx, double dy, double cfl, EulerCtrl* ctrl, int p, cudaStream_t s) {
+  const long long grid = (long long)((nx + kStripW - 1) / kStripW) * ((ny + rows - 1) / rows);
+  auto k = hll ? stream_kernel<T, true, MINB> : stream_kernel<T, false, MINB>;
+  k<<<(unsigned)grid, 32, 0, s>>>(static_cast<const T*>(uin), static_cast<T*>(uout), nx, ny, pitch, plane, (T)dx,
+                                    (T)dy, (T)cfl, rows, ctrl, p);
+  return cudaGetLastError();
+}
+
 template <class T, int TY, int NT, int MINB>
 cudaError_t allow_smem() {
   cudaError_t e = cudaFuncSetAttribute(step_kernel<T, TY, NT, MINB, false>,
@@ -430,32 +618,53 @@ cudaError_t launch_any(int hll, const void* uin, void* uout, int nx, int ny, int
 
 }  // namespace
 
-// Tile shapes (measured at 4096^2, performance build): 32 x 16 cells for fp64
-// and 32 x 32 for fp32, 512 threads, two CTAs (32 warps) per SM at 64
-// registers (shared memory: 92 KB / 83 KB for the four region arrays).
-// Against 32 x 8 (fp64) / 32 x 16 (fp32) tiles of 256 threads at four CTAs
-// per SM: the same occupancy with less halo re-work and half the block
-// barriers per cell (fp64 +15 %, fp32 +17 %).  Measured and not kept at
-// 4096^2: fp64 32 x 12 (-6 %), fp64 32 x 10 with 320 threads at three CTAs
-// per SM (-18 %), fp32 32 x 28 / 32 x 24 at three CTAs per SM (-13 % / -20 %).  fp64 grids whose 32 x 16 tiling fills less than one wave
-// of two CTAs per SM take 32 x 12 tiles (the 500 x 197 shock-bubble: 46.1 ->
-// 41.3 ms).
-constexpr int kThreads = 512;
+// Rows per warp of the streaming kernel: the candidate of least modelled time.
+// With `cap` resident warps per SM and c of them on a scheduler a row takes
+// max(t1, t0 + tc c) (fitted at 200^2 .. 4096^2 over 2 .. 128 rows: within 10 % of
+// the times measured); full waves take the time of cap, the last one that of what
+// is left over.  Few rows cost halo rows, many leave SMs idle.
+struct StreamModel {
+  int cap;
+  double t1, t0, tc;
+};
+constexpr StreamModel kStream64 = {16, 1.03, 0.45, 0.43}, kStream32 = {32, 0.57, 0.14, 0.25};
 
-cudaError_t prepare() {
-  cudaError_t e = allow_smem<double, 16, kThreads, 2>();
-  if (e == cudaSuccess) e = allow_smem<double, 12, kThreads, 2>();
-  if (e == cudaSuccess) e = allow_smem<float, 32, kThreads, 2>();
-  return e;
+int stream_rows(const StreamModel& m, int nx, int ny) {
+  const long long strips = (nx + kStripW - 1) / kStripW;
+  auto row_time = [&](double warps) {  // per SM
+    const double t = m.t0 + m.tc * ((long long)(warps / 4) + ((long long)warps % 4 != 0 || warps != (long long)warps));
+    return warps <= 0 ? 0.0 : (t > m.t1 ? t : m.t1);
+  };
+  int best = 2;
+  double best_t = -1;
+  for (int rows : {2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128}) {
+    const double per_sm = (double)(strips * ((ny + rows - 1) / rows)) / 148.0;
+    const long long full = (long long)(per_sm / m.cap);
+    const double t = (rows + 4) * (full * row_time(m.cap) + row_time(per_sm - (double)full * m.cap));
+    if (best_t < 0 || t < best_t) best_t = t, best = rows;
+  }
+  return best;
 }
+
+// Binary64 grids of at most one wave of 32 x 12 tiles (two 512-thread CTAs per
+// SM) run the shared-memory tile kernel, whose phases spread a step over more
+// threads: 200^2 7.9 us a step against 8.9 streaming, 500 x 197 10.9 against 12.5;
+// past one wave (400^2) 22 against 15.  Binary32 streams at every size (200^2: 6.0
+// against 8.0 us).
+constexpr int kTileH = 12, kThreads = 512;
+
+cudaError_t prepare() { return allow_smem<double, kTileH, kThreads, 2>(); }
 
 cudaError_t step2d(int fp32, int hll, const void* uin, void* uout, int nx, int ny, int pitch, long long plane,
                    double dx, double dy, double cfl, EulerCtrl* ctrl, int p, cudaStream_t s) {
-  if (fp32) return launch_any<float, 32, kThreads, 2>(hll, uin, uout, nx, ny, pitch, plane, dx, dy, cfl, ctrl, p, s);
-  const long long tiles16 = (long long)((nx + TW - 1) / TW) * ((ny + 15) / 16);
-  if (tiles16 < 2 * 148)
-    return launch_any<double, 12, kThreads, 2>(hll, uin, uout, nx, ny, pitch, plane, dx, dy, cfl, ctrl, p, s);
-  return launch_any<double, 16, kThreads, 2>(hll, uin, uout, nx, ny, pitch, plane, dx, dy, cfl, ctrl, p, s);
+  if (fp32)
+    return launch_stream<float, kStream32.cap>(hll, stream_rows(kStream32, nx, ny), uin, uout, nx, ny, pitch, plane,
+                                               dx, dy, cfl, ctrl, p, s);
+  const long long tiles = (long long)((nx + TW - 1) / TW) * ((ny + kTileH - 1) / kTileH);
+  if (tiles <= 2 * 148)
+    return launch_any<double, kTileH, kThreads, 2>(hll, uin, uout, nx, ny, pitch, plane, dx, dy, cfl, ctrl, p, s);
+  return launch_stream<double, kStream64.cap>(hll, stream_rows(kStream64, nx, ny), uin, uout, nx, ny, pitch, plane, dx,
+                                              dy, cfl, ctrl, p, s);
 }
 
 cudaError_t speed2d(int fp32, const void* u, int nx, int ny, int pitch, long long plane, EulerCtrl* ctrl, int slot,
@@ -467,6 +676,19 @@ cudaError_t speed2d(int fp32, const void* u, int nx, int ny, int pitch, long lon
     speed_kernel<float><<<(unsigned)g, 256, 0, s>>>(static_cast<const float*>(u), nx, ny, pitch, plane, ctrl, slot);
   else
     speed_kernel<double><<<(unsigned)g, 256, 0, s>>>(static_cast<const double*>(u), nx, ny, pitch, plane, ctrl, slot);
+  return cudaGetLastError();
+}
+
+cudaError_t prims2d(int fp32, const void* u, int nx, int ny, int pitch, long long plane, void* out, cudaStream_t s) {
+  const long long n = (long long)nx * ny;
+  long long g = (n + 255) / 256;
+  if (g > 148 * 8) g = 148 * 8;
+  if (fp32)
+    prims_kernel<float><<<(unsigned)g, 256, 0, s>>>(static_cast<const float*>(u), nx, ny, pitch, plane,
+                                                    static_cast<float*>(out));
+  else
+    prims_kernel<double><<<(unsigned)g, 256, 0, s>>>(static_cast<const double*>(u), nx, ny, pitch, plane,
+                                                     static_cast<double*>(out));
   return cudaGetLastError();
 }
 
