@@ -13,7 +13,7 @@
 
 #include <cmath>
 
-#include "pmhd/fastmath.hpp"
+#include "fastmath.hpp"
 
 #ifndef __CUDACC__
 #ifndef __host__

@@ -24,7 +24,7 @@
 
 #include <cmath>
 
-#include "pmhd/fastmath.hpp"
+#include "fastmath.hpp"
 
 namespace pmhd {
 
