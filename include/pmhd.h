@@ -94,11 +94,13 @@ typedef struct {
   int steps_per_graph;              /* steps captured per CUDA graph, 0 = auto */
   int autotune;                     /* 1: the first pmhd_advance that runs at least
                                        32 steps times every stage-kernel variant
-                                       (32x19 / 32x8 tiles x resident CTAs per SM)
+                                       (tile shape x resident CTAs per SM)
                                        on 2 live steps each and keeps the fastest
                                        (an ensemble: per grid size, see below);
-                                       results do not depend on the variant.
-                                       0: 32x19 tiles, all resident CTAs.      */
+                                       results do not depend on the variant (up
+                                       to rounding when exact is 0).
+                                       0: 32x19 tiles, of fewer rows on small
+                                       grids, all resident CTAs.               */
 } pmhd_config;
 
 typedef struct {
@@ -116,7 +118,7 @@ typedef struct {
   unsigned long long kernel_launches; /* kernels that did work, total        */
   double device_ms;                 /* GPU time of the last pmhd_advance, from
                                        CUDA events on the handle's stream     */
-  int tile_height;                  /* stage-kernel tile height in use (19, 8) */
+  int tile_height;                  /* cell rows per stage-kernel tile     */
   int ctas;                         /* persistent CTAs per stage launch        */
   unsigned long long zone_cycles;   /* cells x steps of the last advance
                                        (summed over ensemble members)         */

@@ -9,6 +9,7 @@
 // whose stage reports an unusable cell halts alone; the others go on.
 #include <cuda_runtime.h>
 
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -36,8 +37,8 @@ struct pmhd_ensemble {
   Ctrl* hPoll = nullptr;           // pinned, 2n entries: polls one replay behind
   cudaEvent_t evPoll[2] = {nullptr, nullptr};
   Member* dMembers = nullptr;
-  int* dTiles[kNumTileHeights] = {nullptr, nullptr};
-  int* dTile0[kNumTileHeights] = {nullptr, nullptr};
+  int* dTiles[kNumBatchShapes] = {nullptr, nullptr};
+  int* dTile0[kNumBatchShapes] = {nullptr, nullptr};
   Runner run;
   bool tuned = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -127,16 +128,23 @@ double time_type(const pmhd_ensemble* e, double v) {
   return e->cfg.precision == PMHD_FP32 ? (double)(float)v : v;
 }
 
+// Cell rows per tile of shape t for the members `ms`.
+int list_rows(const pmhd_ensemble* e, const std::vector<int>& ms, int t) {
+  std::vector<std::array<int, 2>> sizes;
+  for (int k : ms) sizes.push_back({e->desc[k].nx, e->desc[k].ny});
+  return e->kt->tile_rows(t, reinterpret_cast<const int(*)[2]>(sizes.data()), (int)sizes.size());
+}
+
 // Work list (tile -> member, member -> first tile) of the members `ms` at
 // tile height index t, copied to new device arrays.
 cudaError_t make_work_list(pmhd_ensemble* e, const std::vector<int>& ms, int t, Batch* b, int** d_tiles,
                            int** d_tile0) {
   const int n = (int)e->desc.size();
   std::vector<int> tiles, tile0(n, 0);
+  const int rows = list_rows(e, ms, t);
   for (int k : ms) {
     tile0[k] = (int)tiles.size();
-    const long long nt = (long long)((e->desc[k].nx + 31) / 32) *
-                         ((e->desc[k].ny + kTileHeights[t] - 1) / kTileHeights[t]);
+    const long long nt = num_tiles(e->desc[k].nx, e->desc[k].ny, rows);
     tiles.insert(tiles.end(), (size_t)nt, k);
   }
   *d_tiles = nullptr;
@@ -153,6 +161,7 @@ cudaError_t make_work_list(pmhd_ensemble* e, const std::vector<int>& ms, int t, 
   b->member_tile0 = *d_tile0;
   b->nmembers = n;
   b->ntiles = (int)tiles.size();
+  b->rows = rows;
   return err;
 }
 
@@ -191,7 +200,7 @@ cudaError_t tune_by_size(pmhd_ensemble* e, long long* min_steps, long long* laun
   for (size_t c = 0; c < classes.size() && err == cudaSuccess; c++) {
     float best_ms = -1.f;
     long long steps = 0;
-    for (int t = 0; t < kNumTileHeights && err == cudaSuccess; t++) {
+    for (int t = 0; t < kNumBatchShapes && err == cudaSuccess; t++) {
       LaunchPart part;
       part.ty_idx = t;
       int *dt = nullptr, *d0 = nullptr;
@@ -227,7 +236,7 @@ cudaError_t tune_by_size(pmhd_ensemble* e, long long* min_steps, long long* laun
   }
   // One part per chosen tile height.
   std::vector<LaunchPart> parts;
-  for (int t = 0; t < kNumTileHeights && err == cudaSuccess; t++) {
+  for (int t = 0; t < kNumBatchShapes && err == cudaSuccess; t++) {
     std::vector<int> ms;
     long long top_cells = -1;
     int grid = 0;
@@ -312,7 +321,7 @@ int pmhd_ensemble_destroy(pmhd_ensemble* e) {
   if (e->stream) cudaStreamSynchronize(e->stream);
   e->run.release();
   for (int* d : e->plan_lists) cudaFree(d);
-  for (int t = 0; t < kNumTileHeights; t++) {
+  for (int t = 0; t < kNumBatchShapes; t++) {
     if (e->dTiles[t]) cudaFree(e->dTiles[t]);
     if (e->dTile0[t]) cudaFree(e->dTile0[t]);
   }
@@ -407,14 +416,15 @@ int pmhd_ensemble_create(const pmhd_config* common, const pmhd_member_desc* memb
       cudaMemcpyAsync(e->dMembers, e->hm.data(), sizeof(Member) * n, cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     rc = PMHD_ERR_CUDA;
   // Work lists: each member's tiles, members in order, per tile height.
-  std::vector<int> tiles, tile0;
-  for (int t = 0; rc == PMHD_OK && t < kNumTileHeights; t++) {
+  std::vector<int> tiles, tile0, all(n);
+  for (int k = 0; k < n; k++) all[k] = k;
+  for (int t = 0; rc == PMHD_OK && t < kNumBatchShapes; t++) {
     tiles.clear();
     tile0.assign(n, 0);
+    const int rows = list_rows(e, all, t);
     for (int k = 0; k < n; k++) {
       tile0[k] = (int)tiles.size();
-      const long long nt =
-          (long long)((members[k].nx + 31) / 32) * ((members[k].ny + kTileHeights[t] - 1) / kTileHeights[t]);
+      const long long nt = num_tiles(members[k].nx, members[k].ny, rows);
       if ((long long)tiles.size() + nt > (long long)INT_MAX) {
         rc = PMHD_ERR_UNSUPPORTED;
         break;
@@ -440,6 +450,7 @@ int pmhd_ensemble_create(const pmhd_config* common, const pmhd_member_desc* memb
     b.member_tile0 = e->dTile0[t];
     b.nmembers = n;
     b.ntiles = (int)tiles.size();
+    b.rows = rows;
   }
   e->run.kt = e->kt;
   e->run.precision = common->precision;
@@ -595,7 +606,7 @@ int pmhd_ensemble_advance(pmhd_ensemble* e, long long max_steps, pmhd_stats* tot
     if (mst != PMHD_OK || !e->failed[k]) st.status = mst;
     st.zone_cycles = (unsigned long long)done * (unsigned long long)d.nx * d.ny;
     st.device_ms = ms;
-    st.tile_height = kTileHeights[e->run.parts.empty() ? e->run.choice.ty_idx : e->member_ty[k]];
+    st.tile_height = tile_height(e->run.parts.empty() ? e->run.choice.ty_idx : e->member_ty[k]);
     if (mst != PMHD_OK && status == PMHD_OK) {
       status = mst;
       tot.bad_i = st.bad_i;
@@ -632,7 +643,7 @@ int pmhd_ensemble_advance(pmhd_ensemble* e, long long max_steps, pmhd_stats* tot
     const int def = sms * e->kt->ctas_per_sm(e->cfg.precision, e->run.hlld, plan[top].ty_idx, 1);
     const int g = plan[top].grid > 0 ? plan[top].grid : def;
     const int nt = plan[top].batch.ntiles;
-    tot.tile_height = kTileHeights[plan[top].ty_idx];
+    tot.tile_height = tile_height(plan[top].ty_idx);
     tot.ctas = g < nt ? g : nt;
   }
   for (int k = 0; k < n; k++) e->mstats[k].ctas = tot.ctas;

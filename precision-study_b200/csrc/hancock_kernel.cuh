@@ -407,7 +407,8 @@ __global__ void __launch_bounds__(256, HancockTileOf<Pol>::MINB)
   using HT = HancockTileOf<Pol>;
   constexpr int TYH = HT::TYH;
   static_assert(TYH == 8, "the region box is the 32 x 8 stage-kernel descriptor's");
-  constexpr int TI = kTileHeights[0] == 8 ? 0 : 1;  // index of the 32 x 8 descriptors in Member::tm
+  constexpr int TI = 1;  // index of the 32 x 8 descriptors in Member::tm
+  static_assert(kTileShapes[TI] == 8, "32 x 8 descriptors");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   HT& s = *reinterpret_cast<HT*>(smem_raw);
   __shared__ __align__(8) uint64_t bar;

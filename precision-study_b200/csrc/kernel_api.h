@@ -24,13 +24,21 @@ struct Ctrl;
 
 enum Precision : int { PREC_FP64 = 0, PREC_FP32 = 1, PREC_MIXED = 2 };
 
-// Tile heights compiled into the library (tile width is 32).  Index into
-// Member::tm and the Batch tile tables; index 0 is the default.
+// Tile shapes compiled into the library (tile width is 32), as the tile height
+// plus kSplit for the shapes whose x and y interfaces go to separate warps.
+// Index into Member::tm and the Batch tile tables; index 0 is the default.  Every
+// precision has the first kNumBatchShapes, which are also the ones batches
+// (ensembles) run; the performance build's binary64 and binary32 kernels have
+// them all (single grids).
 #ifndef PMHD_TY0
 #define PMHD_TY0 19
 #endif
-constexpr int kTileHeights[2] = {PMHD_TY0, 8};
-constexpr int kNumTileHeights = 2;
+constexpr int kSplit = 64;
+constexpr int kNumTileShapes = 5, kNumBatchShapes = 2;
+constexpr int kTileShapes[kNumTileShapes] = {PMHD_TY0, 8, 8 + kSplit, 4 + kSplit, 2 + kSplit};
+constexpr int tile_height(int idx) { return kTileShapes[idx] & (kSplit - 1); }
+// Tiles of `rows` cell rows an nx x ny grid has.
+inline long long num_tiles(int nx, int ny, int rows) { return (long long)((nx + 31) / 32) * ((ny + rows - 1) / rows); }
 // A batched stage launch hands its CTAs runs of consecutive tiles, at most
 // this many (a power of two; see batch_run in kernels.cu).
 constexpr int kBatchRunMax = 16;
@@ -38,7 +46,7 @@ constexpr int kBatchRunMax = 16;
 // One grid of a batch; lives in device memory (64-byte aligned for the TMA
 // descriptors).
 struct alignas(64) Member {
-  CUtensorMap tm[kNumTileHeights][2];  // [tile height][U, U1]: stage-1 / stage-2 inputs
+  CUtensorMap tm[kNumTileShapes][2];  // [tile shape][U, U1]: stage-1 / stage-2 inputs
   void* u;            // U planes (stage-1 input, stage-2 output)
   void* u1;           // U1 planes (stage-1 output, stage-2 input)
   Ctrl* ctrl;         // this grid's control block
@@ -51,13 +59,15 @@ struct alignas(64) Member {
   double inv_dx, inv_dy;      // 1 / dx, 1 / dy divided in the precision's time type
 };
 
-// The work list of one tile height.
+// The work list of one tile shape.  Its tiles may cover fewer rows than the shape
+// has (same kernel, the warps of the other rows idle): see tile_rows in kernels.cu.
 struct Batch {
   const Member* members;   // device array of nmembers
   const int* tile_member;  // device array: global tile -> member (nullptr: all tiles are member 0)
   const int* member_tile0; // device array: first global tile of each member (nullptr: 0)
   int nmembers;
   int ntiles;
+  int rows;                // cell rows a tile covers: at most the shape's height
 };
 
 struct KernelTable {
@@ -65,7 +75,7 @@ struct KernelTable {
   // Sets dynamic shared-memory limits; call once per process and device.
   cudaError_t (*init)();
   // One SSPRK2 stage (1 or 2) over every member of the batch.  `ty_idx`
-  // selects the tile height (kTileHeights), `grid` the number of persistent
+  // selects the tile shape (kTileShapes), `grid` the number of persistent
   // CTAs (<= 0: SM count x resident CTAs), `parity` the step's Ctrl slot.
   // `single` != nullptr: a one-grid batch whose member is passed by value
   // (host copy; only b.ntiles is used); nullptr: the members of `b`.
@@ -81,8 +91,12 @@ struct KernelTable {
                             int pitch, const int bc[4], cudaStream_t s);
   cudaError_t (*soa_to_aos)(int precision, const void* u, long long plane, int nx, int ny, int pitch, int layout,
                             void* aos, cudaStream_t s);
-  // Shared memory per CTA of the stage kernel with tile height kTileHeights[ty_idx].
-  size_t (*stage_smem)(int precision, int ty_idx);
+  // Whether single grids of a precision can run a tile shape, and the one they
+  // run by default (indices into kTileShapes).
+  bool (*has_shape)(int precision, int idx);
+  int (*default_shape)(int precision, int nx, int ny);
+  // Cell rows per tile of shape idx for one or more grids (nx, ny) in a launch.
+  int (*tile_rows)(int idx, const int (*sizes)[2], int n);
   // One MUSCL-Hancock step of a single grid: part 0 = the control prologue,
   // part 1 = the step (reads m.u for parity 0 / m.u1 for parity 1, writes
   // the other).  fp64 and fp32 only.

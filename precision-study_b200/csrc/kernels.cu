@@ -13,10 +13,20 @@ namespace PMHD_KNS {
 
 #include "hancock_kernel.cuh"  // no includes of its own; lives in this namespace
 
+// 32 x 19 tiles may cover fewer rows (tile_rows).
+template <int TY>
+constexpr bool kPartial = TY == kTileShapes[0];
+
 template <class Pol, int STAGE, bool HLLD, int TY, bool BATCHED>
 static cudaError_t set_smem_attr() {
-  return cudaFuncSetAttribute(stage_kernel<Pol, STAGE, HLLD, TY, BATCHED>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<Pol, TY>::total);
+  cudaError_t e = cudaFuncSetAttribute(stage_kernel<Pol, STAGE, HLLD, TY, BATCHED, false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<Pol, TY>::total);
+  if constexpr (kPartial<TY>) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(stage_kernel<Pol, STAGE, HLLD, TY, BATCHED, true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<Pol, TY>::total);
+  }
+  return e;
 }
 
 template <class Pol, int TY, bool BATCHED>
@@ -34,11 +44,20 @@ static cudaError_t init_pol_ty() {
   return e != cudaSuccess ? e : init_pol_ty_b<Pol, TY, true>();
 }
 
+// The policy has the shapes past kNumBatchShapes.
+template <class Pol>
+constexpr bool kAllShapes = PMHD_FAST_FLUX != 0 && !Pol::kMixed;
+
 template <class Pol>
 static cudaError_t init_pol() {
   cudaError_t e;
-  if ((e = init_pol_ty<Pol, kTileHeights[0]>()) != cudaSuccess) return e;
-  return init_pol_ty<Pol, kTileHeights[1]>();
+  if ((e = init_pol_ty<Pol, kTileShapes[0]>()) != cudaSuccess) return e;
+  if constexpr (kAllShapes<Pol>) {
+    if ((e = init_pol_ty_b<Pol, kTileShapes[2], false>()) != cudaSuccess) return e;
+    if ((e = init_pol_ty_b<Pol, kTileShapes[3], false>()) != cudaSuccess) return e;
+    if ((e = init_pol_ty_b<Pol, kTileShapes[4], false>()) != cudaSuccess) return e;
+  }
+  return init_pol_ty<Pol, kTileShapes[1]>();
 }
 
 template <class Pol, bool HLLD>
@@ -80,7 +99,7 @@ static int occupancy() {
   std::lock_guard<std::mutex> lk(mu);
   if (per_sm < 0) {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stage_kernel<Pol, 1, HLLD, TY, BATCHED>, Geo<TY>::NT,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stage_kernel<Pol, 1, HLLD, TY, BATCHED, false>, Geo<TY>::NT,
                                                   Smem<Pol, TY>::total);
     per_sm = nb > 0 ? nb : 1;
   }
@@ -104,55 +123,64 @@ static int batch_run(int ntiles, int grid) {
 }
 
 template <class Pol, bool HLLD, int TY, bool BATCHED>
-static void launch_one(int stage, const Batch& b, const Member& m0, int parity, int run, int grid, cudaStream_t s) {
+static cudaError_t launch_one(int stage, const Batch& b, const Member& m0, int parity, int run, int grid,
+                              cudaStream_t s) {
   const size_t smem = Smem<Pol, TY>::total;
-  if (stage == 1)
-    stage_kernel<Pol, 1, HLLD, TY, BATCHED><<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run);
-  else
-    stage_kernel<Pol, 2, HLLD, TY, BATCHED><<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run);
+  auto go = [&](auto* kernel) {
+    kernel<<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run);
+    return cudaGetLastError();
+  };
+  if constexpr (kPartial<TY>) {
+    if (b.rows < tile_height(0))
+      return go(stage == 1 ? stage_kernel<Pol, 1, HLLD, TY, BATCHED, true> : stage_kernel<Pol, 2, HLLD, TY, BATCHED, true>);
+  }
+  return go(stage == 1 ? stage_kernel<Pol, 1, HLLD, TY, BATCHED, false> : stage_kernel<Pol, 2, HLLD, TY, BATCHED, false>);
 }
 
-template <class Pol, int TY>
+template <class Pol, int TY, bool BATCHES>
 static int occ_pol_ty(int hlld, bool batched) {
-  if (batched) return hlld ? occupancy<Pol, true, TY, true>() : occupancy<Pol, false, TY, true>();
+  if constexpr (BATCHES)
+    if (batched) return hlld ? occupancy<Pol, true, TY, true>() : occupancy<Pol, false, TY, true>();
   return hlld ? occupancy<Pol, true, TY, false>() : occupancy<Pol, false, TY, false>();
 }
 
-template <class Pol, int TY>
+template <class Pol, int TY, bool BATCHES>
 static cudaError_t launch_stage_pol(int hlld, int stage, const Batch& b, const Member* single, int parity, int grid,
                                     cudaStream_t s) {
   if (b.ntiles <= 0) return cudaSuccess;
   const bool batched = single == nullptr;
-  if (grid <= 0) grid = sm_count() * occ_pol_ty<Pol, TY>(hlld, batched);
+  if (batched && !BATCHES) return cudaErrorNotSupported;
+  if (grid <= 0) grid = sm_count() * occ_pol_ty<Pol, TY, BATCHES>(hlld, batched);
   const int run = batched ? batch_run(b.ntiles, grid) : 1;
   const int units = (b.ntiles + run - 1) / run;  // runs of tiles
   if (grid > units) grid = units;
   static const Member empty = {};
   const Member& m0 = batched ? empty : *single;
-  if (hlld) {
-    if (batched)
-      launch_one<Pol, true, TY, true>(stage, b, m0, parity, run, grid, s);
-    else
-      launch_one<Pol, true, TY, false>(stage, b, m0, parity, run, grid, s);
-  } else {
-    if (batched)
-      launch_one<Pol, false, TY, true>(stage, b, m0, parity, run, grid, s);
-    else
-      launch_one<Pol, false, TY, false>(stage, b, m0, parity, run, grid, s);
+  if constexpr (BATCHES) {
+    if (batched) {
+      return hlld ? launch_one<Pol, true, TY, true>(stage, b, m0, parity, run, grid, s)
+                  : launch_one<Pol, false, TY, true>(stage, b, m0, parity, run, grid, s);
+    }
   }
-  return cudaGetLastError();
+  return hlld ? launch_one<Pol, true, TY, false>(stage, b, m0, parity, run, grid, s)
+              : launch_one<Pol, false, TY, false>(stage, b, m0, parity, run, grid, s);
 }
 
 template <class Pol>
 static cudaError_t launch_stage_ty(int hlld, int stage, int ty_idx, const Batch& b, const Member* single, int parity,
                                    int grid, cudaStream_t s) {
-  return ty_idx == 0 ? launch_stage_pol<Pol, kTileHeights[0]>(hlld, stage, b, single, parity, grid, s)
-                     : launch_stage_pol<Pol, kTileHeights[1]>(hlld, stage, b, single, parity, grid, s);
+  if (ty_idx == 0) return launch_stage_pol<Pol, kTileShapes[0], true>(hlld, stage, b, single, parity, grid, s);
+  if (ty_idx == 1) return launch_stage_pol<Pol, kTileShapes[1], true>(hlld, stage, b, single, parity, grid, s);
+  if constexpr (kAllShapes<Pol>) {
+    if (ty_idx == 2) return launch_stage_pol<Pol, kTileShapes[2], false>(hlld, stage, b, single, parity, grid, s);
+    if (ty_idx == 3) return launch_stage_pol<Pol, kTileShapes[3], false>(hlld, stage, b, single, parity, grid, s);
+    if (ty_idx == 4) return launch_stage_pol<Pol, kTileShapes[4], false>(hlld, stage, b, single, parity, grid, s);
+  }
+  return cudaErrorNotSupported;
 }
 
 static cudaError_t launch_stage(int precision, int hlld, int stage, int ty_idx, const Batch& b, const Member* single,
                                 int parity, int grid, cudaStream_t s) {
-  if (ty_idx < 0 || ty_idx >= kNumTileHeights) return cudaErrorInvalidValue;
   switch (precision) {
     case PREC_FP64: return launch_stage_ty<PolF64>(hlld, stage, ty_idx, b, single, parity, grid, s);
     case PREC_FP32: return launch_stage_ty<PolF32>(hlld, stage, ty_idx, b, single, parity, grid, s);
@@ -163,8 +191,13 @@ static cudaError_t launch_stage(int precision, int hlld, int stage, int ty_idx, 
 
 template <class Pol>
 static int occ_pol(int hlld, int ty_idx, bool batched) {
-  return ty_idx == 0 ? occ_pol_ty<Pol, kTileHeights[0]>(hlld, batched)
-                     : occ_pol_ty<Pol, kTileHeights[1]>(hlld, batched);
+  if constexpr (kAllShapes<Pol>) {
+    if (ty_idx == 2) return occ_pol_ty<Pol, kTileShapes[2], false>(hlld, batched);
+    if (ty_idx == 3) return occ_pol_ty<Pol, kTileShapes[3], false>(hlld, batched);
+    if (ty_idx == 4) return occ_pol_ty<Pol, kTileShapes[4], false>(hlld, batched);
+  }
+  return ty_idx == 0 ? occ_pol_ty<Pol, kTileShapes[0], true>(hlld, batched)
+                     : occ_pol_ty<Pol, kTileShapes[1], true>(hlld, batched);
 }
 
 static int ctas_per_sm(int precision, int hlld, int ty_idx, int batched) {
@@ -175,13 +208,41 @@ static int ctas_per_sm(int precision, int hlld, int ty_idx, int batched) {
   }
 }
 
-static size_t stage_smem(int precision, int ty_idx) {
-  const bool t8 = ty_idx == 0;
-  switch (precision) {
-    case PREC_FP64: return t8 ? Smem<PolF64, kTileHeights[0]>::total : Smem<PolF64, kTileHeights[1]>::total;
-    case PREC_FP32: return t8 ? Smem<PolF32, kTileHeights[0]>::total : Smem<PolF32, kTileHeights[1]>::total;
-    default: return t8 ? Smem<PolMixed, kTileHeights[0]>::total : Smem<PolMixed, kTileHeights[1]>::total;
-  }
+// Tile shape of a single grid: the smallest split shape that gives every tile an SM
+// of its own, if there is one (a stage is then one tile's dependent chain; 64^2
+// binary64, us a step: 33 with 32 x 19 tiles, 20 / 14 / 12 with split 32 x 8 / 4 / 2;
+// 192^2: 34 and 20 with split 32 x 8), else 32 x 19.  Only the performance
+// build's binary64: the compiler contracts binary32 fluxes differently for every
+// shape, and binary32 and mixed results of grids and ensembles stay together.
+static int default_shape(int precision, int nx, int ny) {
+  if (!PMHD_FAST_FLUX || precision != PREC_FP64) return 0;
+  for (int idx = kNumTileShapes - 1; idx >= kNumBatchShapes; idx--)
+    if (num_tiles(nx, ny, tile_height(idx)) <= sm_count()) return idx;
+  return 0;
+}
+
+// Cell rows per tile of a list of grids: the fewest with which the persistent
+// CTAs, one per SM, take no more rounds than with full 32 x 19 tiles -- a tile's
+// time falls with its rows, and the SMs a short last round leaves idle take part.
+// The bits do not depend on it.  Mixed, us a step, against full tiles: 64^2 14.6 /
+// 22.4, 128^2 16.1 / 22.4, 320^2 32.0 / 38.2.
+static int tile_rows(int idx, const int (*sizes)[2], int n) {
+  const int height = tile_height(idx);
+  if (idx != 0) return height;
+  auto tiles = [&](int rows) {
+    long long t = 0;
+    for (int k = 0; k < n; k++) t += num_tiles(sizes[k][0], sizes[k][1], rows);
+    return t;
+  };
+  const long long sms = sm_count(), budget = (tiles(height) + sms - 1) / sms * sms;
+  for (int rows = 2; rows < height; rows++)
+    if (tiles(rows) <= budget) return rows;
+  return height;
+}
+
+static bool has_shape(int precision, int idx) {
+  return idx >= 0 && (idx < kNumBatchShapes || (idx < kNumTileShapes && PMHD_FAST_FLUX &&
+                                                (precision == PREC_FP64 || precision == PREC_FP32)));
 }
 
 static int grid_for(long long n) {
@@ -286,7 +347,8 @@ const KernelTable& PMHD_TABLE_FN(PMHD_KNS)() {
   static const KernelTable t = {PMHD_STR(PMHD_KNS),          PMHD_KNS::init,
                                 PMHD_KNS::launch_stage,      PMHD_KNS::ctas_per_sm,
                                 PMHD_KNS::launch_speed,      PMHD_KNS::launch_aos_to_soa,
-                                PMHD_KNS::launch_soa_to_aos, PMHD_KNS::stage_smem,
+                                PMHD_KNS::launch_soa_to_aos, PMHD_KNS::has_shape,         PMHD_KNS::default_shape,
+                                PMHD_KNS::tile_rows,
                                 PMHD_KNS::launch_hancock};
   return t;
 }

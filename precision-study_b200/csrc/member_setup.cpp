@@ -41,8 +41,8 @@ bool encode_member_tmaps(Member& m, size_t elem) {
   const cuuint64_t strides[2] = {(cuuint64_t)m.pitch * elem, (cuuint64_t)m.plane * elem};
   const cuuint32_t estr[3] = {1, 1, 1};
   void* bufs[2] = {m.u, m.u1};
-  for (int t = 0; t < kNumTileHeights; t++) {
-    const cuuint32_t box[3] = {32 + 4, (cuuint32_t)kTileHeights[t] + 4, 9};
+  for (int t = 0; t < kNumTileShapes; t++) {
+    const cuuint32_t box[3] = {32 + 4, (cuuint32_t)tile_height(t) + 4, 9};
     for (int k = 0; k < 2; k++) {
       CUresult r = enc(&m.tm[t][k], elem == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                        bufs[k], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,

@@ -161,7 +161,10 @@ extern "C" int pmhd_advance_noalloc(const pmhd_config* cfg, const void* d_in, vo
   batch.tile_member = nullptr;
   batch.member_tile0 = nullptr;
   batch.nmembers = 1;
-  batch.ntiles = ((nx + 31) / 32) * ((ny + kTileHeights[0] - 1) / kTileHeights[0]);
+  const int shape = kt.default_shape(cfg->precision, nx, ny);  // as pmhd_create
+  const int size[1][2] = {{nx, ny}};
+  batch.rows = kt.tile_rows(shape, size, 1);
+  batch.ntiles = (int)num_tiles(nx, ny, batch.rows);
 
   // Values the reference holds in its Real type.
   auto tt = [&](double v) { return f32 ? (double)(float)v : v; };
@@ -189,8 +192,8 @@ extern "C" int pmhd_advance_noalloc(const pmhd_config* cfg, const void* d_in, vo
   auto launch_pairs = [&](long long pairs) -> int {
     for (long long q = 0; q < pairs; q++)
       for (int par = 0; par < 2; par++) {
-        if (kt.stage(cfg->precision, hlld, 1, 0, batch, &hm, par, 0, s) != cudaSuccess) return PMHD_ERR_CUDA;
-        if (kt.stage(cfg->precision, hlld, 2, 0, batch, &hm, par, 0, s) != cudaSuccess) return PMHD_ERR_CUDA;
+        if (kt.stage(cfg->precision, hlld, 1, shape, batch, &hm, par, 0, s) != cudaSuccess) return PMHD_ERR_CUDA;
+        if (kt.stage(cfg->precision, hlld, 2, shape, batch, &hm, par, 0, s) != cudaSuccess) return PMHD_ERR_CUDA;
       }
     return PMHD_OK;
   };

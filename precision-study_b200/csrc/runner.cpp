@@ -67,7 +67,8 @@ cudaError_t Runner::tune(int steps, TuneResult* res) {
   float best_ms = -1.f, default_ms = -1.f;
   int ncand = 0;
   cudaError_t err = cudaSuccess;
-  for (int ty = 0; ty < kNumTileHeights && err == cudaSuccess; ty++) {
+  for (int ty = 0; ty < kNumTileShapes && err == cudaSuccess; ty++) {
+    if (!kt->has_shape(precision, ty) || (!single && ty >= kNumBatchShapes)) continue;
     const int occ = kt->ctas_per_sm(precision, hlld, ty, single == nullptr);
     for (int k = occ; k >= 1 && err == cudaSuccess; k--) {
       choice.ty_idx = ty;

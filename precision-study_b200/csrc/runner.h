@@ -15,7 +15,7 @@ namespace pmhd {
 
 // Which compiled stage-kernel variant runs and with how many persistent CTAs.
 struct LaunchChoice {
-  int ty_idx = 0;  // index into kTileHeights
+  int ty_idx = 0;  // index into kTileShapes
   int grid = 0;    // persistent CTAs; 0 = SM count x resident CTAs
 };
 
@@ -40,7 +40,7 @@ class Runner {
   int precision = 0;
   int hlld = 1;
   cudaStream_t stream = nullptr;
-  Batch batch[kNumTileHeights];
+  Batch batch[kNumTileShapes];
   const Member* single = nullptr;  // host copy of a one-grid batch's member, or nullptr
   LaunchChoice choice;
   // Multi-part plan: when non-empty, a step launches stage 1 of every part,

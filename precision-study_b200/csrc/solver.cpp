@@ -274,13 +274,16 @@ int pmhd_create(const pmhd_config* cfg, pmhd_solver** out) {
     s->run.hlld = cfg->solver == PMHD_SOLVER_HLLD ? 1 : 0;
     s->run.hancock = cfg->order == PMHD_ORDER_HANCOCK ? 1 : 0;
     s->run.stream = s->stream;
-    for (int t = 0; t < kNumTileHeights; t++) {
+    s->run.choice.ty_idx = s->kt->default_shape(cfg->precision, cfg->nx, cfg->ny);
+    for (int t = 0; t < kNumTileShapes; t++) {
       Batch& b = s->run.batch[t];
       b.members = s->dMember;
       b.tile_member = nullptr;
       b.member_tile0 = nullptr;
       b.nmembers = 1;
-      b.ntiles = ((cfg->nx + 31) / 32) * ((cfg->ny + kTileHeights[t] - 1) / kTileHeights[t]);
+      const int size[1][2] = {{cfg->nx, cfg->ny}};
+      b.rows = s->kt->tile_rows(t, size, 1);
+      b.ntiles = (int)num_tiles(cfg->nx, cfg->ny, b.rows);
     }
   }
   if (rc == PMHD_OK && cudaStreamSynchronize(s->stream) != cudaSuccess) rc = PMHD_ERR_CUDA;
@@ -522,7 +525,7 @@ int pmhd_advance(pmhd_solver* s, double t_end, long long max_steps, pmhd_stats* 
   s->stats.status = status;
   s->stats.device_ms = ms;
   s->stats.zone_cycles = (unsigned long long)done_steps * (unsigned long long)s->cfg.nx * s->cfg.ny;
-  s->stats.tile_height = kTileHeights[s->run.choice.ty_idx];
+  s->stats.tile_height = s->run.batch[s->run.choice.ty_idx].rows;
   {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->cfg.device);

@@ -82,21 +82,31 @@ constexpr int TX = 32;                    // tile width: one warp per tile row
 constexpr int NTA = 256;                  // threads per CTA of the auxiliary kernels
 constexpr uint32_t kWaitIters = 1u << 22; // bound on mbarrier polls
 
-// Geometry of a 32 x TY tile: TY warps own one tile row each, one more warp
-// handles the tile's bottom row of y-interfaces and left column of
-// x-interfaces.
-template <int TY_>
+// Index of a shape in kTileShapes / Member::tm.
+constexpr int shape_index(int sh) {
+  for (int k = 0; k < kNumTileShapes; k++)
+    if (kTileShapes[k] == sh) return k;
+  return -1;
+}
+
+// Geometry of a tile shape SH, 32 x TY cells.  TY warps own one tile row each,
+// one more warp handles the tile's bottom row of y-interfaces and left column of
+// x-interfaces; each runs two rounds of one direction.  Split shapes give every
+// round a warp of its own: TY warps the x-interfaces, TY the y-interfaces, one the
+// bottom row, one the left column.
+template <int SH>
 struct Geo {
-  static constexpr int TY = TY_;
-  static constexpr int HX = TX + 4, HY = TY + 4;  // tile with halo
-  static constexpr int TC = HX * HY;              // cells per loaded tile
-  static constexpr int NW = TY + 1;               // warps per CTA
-  static constexpr int NT = NW * 32;              // threads per CTA
-  static constexpr int FXN = TY * (TX + 1);       // x-interfaces per tile
-  static constexpr int GYN = (TY + 1) * TX;       // y-interfaces per tile
+  static constexpr int TY = SH & (kSplit - 1);
+  static constexpr bool SPLIT = (SH & kSplit) != 0;
+  static constexpr int INDEX = shape_index(SH);
+  static constexpr int HX = TX + 4, HY = TY + 4;       // tile with halo
+  static constexpr int TC = HX * HY;                   // cells per loaded tile
+  static constexpr int NW = SPLIT ? 2 * TY + 2 : TY + 1;  // warps per CTA
+  static constexpr int NT = NW * 32;                   // threads per CTA
+  static constexpr int FXN = TY * (TX + 1);            // x-interfaces per tile
+  static constexpr int GYN = (TY + 1) * TX;            // y-interfaces per tile
   static_assert(TY <= 32, "the extra warp covers the left column");
 };
-
 constexpr size_t align128(size_t b) { return (b + 127) & ~size_t(127); }
 
 // Per-policy, per-tile-height launch tuning, measured on B200 at Orszag-Tang
@@ -141,7 +151,7 @@ struct Tune {
   static constexpr int minb_r32 = Pol::kMixed ? 2 : 3;
 #endif
   static constexpr int minb8 = r64 ? minb_r64 : minb_r32;
-  static constexpr int minb = TY == 8 ? minb8 : (TY == 4 ? (minb8 * 9) / 5 : 1);
+  static constexpr int minb = TY == 8 ? minb8 : 1;
 };
 
 template <class Pol, int TY>
@@ -494,16 +504,17 @@ __device__ __forceinline__ bool member_active(const Member& m, int p) {
 // scalars are then constant-bank operands and its TMA descriptors live in
 // parameter space); `b` only supplies the tile count.  BATCHED = true: the
 // members of `b`, read from device memory per tile, handed out in runs of
-// `run` (a power of two) consecutive tiles.
-template <class Pol, int STAGE, bool HLLD, int TY, bool BATCHED>
+// `run` (a power of two) consecutive tiles.  PARTIAL = true: tiles cover b.rows
+// rows of the shape's (a runtime height costs 2 % on large grids).
+template <class Pol, int STAGE, bool HLLD, int TY, bool BATCHED, bool PARTIAL>
 __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
     stage_kernel(const __grid_constant__ Member m0, const Batch b, const int p, const int run) {
   using S = typename Pol::S;
   using R = typename Pol::R;
   using G = Geo<TY>;
-  constexpr int HX = G::HX, TC = G::TC, NT = G::NT, FXN = G::FXN, GYN = G::GYN;
+  constexpr int TYT = G::TY, HX = G::HX, TC = G::TC, NT = G::NT, FXN = G::FXN, GYN = G::GYN;
   constexpr int NBUF = Tune<Pol, TY>::nbuf;
-  constexpr int TI = kTileHeights[0] == TY ? 0 : 1;  // index into Member::tm
+  constexpr int TI = G::INDEX;  // index into Member::tm
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* sP = reinterpret_cast<R*>(smem_raw + Smem<Pol, TY>::p_off);
   R* sFx = reinterpret_cast<R*>(smem_raw + Smem<Pol, TY>::fx_off);
@@ -511,6 +522,7 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
   __shared__ __align__(8) uint64_t bar[NBUF];
   auto ubuf = [&](int k) { return reinterpret_cast<S*>(smem_raw + (size_t)k * Smem<Pol, TY>::u_stride); };
 
+  const int rows = PARTIAL ? b.rows : TYT;  // of a tile
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   auto member_of = [&](int t) { return BATCHED ? b.tile_member[t] : 0; };
@@ -562,7 +574,7 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
     const int lt = t - tile0_of(mi);
     const int tiles_x = (mm.nx + TX - 1) / TX;
     mbar_arrive_expect_tx(&bar[k], (uint32_t)Smem<Pol, TY>::u_bytes);
-    tma_load_3d(ubuf(k), &mm.tm[TI][STAGE - 1], &bar[k], (lt % tiles_x) * TX, (lt / tiles_x) * TY, 0);
+    tma_load_3d(ubuf(k), &mm.tm[TI][STAGE - 1], &bar[k], (lt % tiles_x) * TX, (lt / tiles_x) * rows, 0);
   };
 
   if (tid == 0) {
@@ -587,7 +599,7 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
     }
     const int lt = tile - tile0_of(mi);
     const int tiles_x = (m.nx + TX - 1) / TX;
-    const int i0 = (lt % tiles_x) * TX, j0 = (lt / tiles_x) * TY;
+    const int i0 = (lt % tiles_x) * TX, j0 = (lt / tiles_x) * rows;
     const Phys<R> phR = Phys<R>::make(m.gamma, m.tol);
     const Phys<S> phS = Phys<S>::make(m.gamma, m.tol);
     const int cb = it % NBUF;                        // buffer of this tile
@@ -606,9 +618,9 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
     // First order needs no primitives (but for the lean binary64 flux): the
     // conserved states are staged.
     bool usable = true;  // performance build: this thread's cells (cell_usable_fast)
-    for (int q = tid; q < TC; q += NT) {
+    for (int q = tid; q < HX * (rows + 4); q += NT) {
       const int cx = q % HX, cy = q / HX;
-      if ((cx < 2 || cx >= TX + 2) && (cy < 2 || cy >= TY + 2)) continue;
+      if ((cx < 2 || cx >= TX + 2) && (cy < 2 || cy >= rows + 2)) continue;
       S U9[NVAR], P9[NVAR];
 #pragma unroll
       for (int k = 0; k < NVAR; k++) U9[k] = sU[k * TC + q];
@@ -647,9 +659,15 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
     // direction for the whole warp, through one (not unrolled) copy of the
     // flux code.
 #pragma unroll 1
-    for (int r = 0; r < 2; r++) {
+    for (int r = 0; r < (G::SPLIT ? 1 : 2); r++) {
       int axis, fx, fy;
-      if (warp < TY) {
+      if constexpr (G::SPLIT) {
+        axis = warp >= TYT && warp <= 2 * TYT;
+        fx = axis ? lane : (warp < TYT ? lane + 1 : 0);
+        fy = warp < TYT ? warp : (warp < 2 * TYT ? warp - TYT + 1 : (warp == 2 * TYT ? 0 : lane));
+        if (warp == 2 * TYT + 1 && lane >= TYT) continue;
+      } else if (warp < TYT) {
+        if (warp >= rows) continue;
         axis = r;
         fx = r ? lane : lane + 1;
         fy = r ? warp + 1 : warp;
@@ -657,7 +675,7 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
         axis = 1 - r;
         fx = r ? 0 : lane;
         fy = r ? lane : 0;
-        if (r == 1 && lane >= TY) continue;
+        if (r == 1 && lane >= rows) continue;
       }
       // x: interface between cells (i0+fx-1, j0+fy) and (i0+fx, j0+fy)
       // y: interface between cells (i0+fx, j0+fy-1) and (i0+fx, j0+fy)
@@ -704,7 +722,7 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
     // ---- divergence, update, checks, store, next-step speed ---------------
     const int tx = lane, ty = warp;
     const int gi = i0 + tx, gj = j0 + ty;
-    if (warp < TY && gi < m.nx && gj < m.ny) {
+    if (warp < rows && gi < m.nx && gj < m.ny) {
       const size_t gidx = (size_t)(gj + GHOST) * m.pitch + (gi + GHOST);
       const int lc = (ty + 2) * HX + tx + 2;
       const S* u_in = static_cast<const S*>(STAGE == 1 ? m.u : m.u1);
