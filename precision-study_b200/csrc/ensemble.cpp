@@ -372,7 +372,7 @@ int pmhd_ensemble_create(const pmhd_config* common, const pmhd_member_desc* memb
   e->failed.assign(n, 0);
   e->member_ty.assign(n, 0);
   int rc = PMHD_OK;
-  if (e->kt->init() != cudaSuccess) rc = PMHD_ERR_CUDA;
+  if (e->kt->init(common->precision) != cudaSuccess) rc = PMHD_ERR_CUDA;
   // Layout of the member states.
   e->hm.assign(n, Member());
   e->state_off.assign(n, 0);

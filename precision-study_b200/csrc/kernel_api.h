@@ -72,8 +72,9 @@ struct Batch {
 
 struct KernelTable {
   const char* name;
-  // Sets dynamic shared-memory limits; call once per process and device.
-  cudaError_t (*init)();
+  // Sets the dynamic shared-memory limits of a precision's kernels (and so loads
+  // them); call once per process and device.
+  cudaError_t (*init)(int precision);
   // One SSPRK2 stage (1 or 2) over every member of the batch.  `ty_idx`
   // selects the tile shape (kTileShapes), `grid` the number of persistent
   // CTAs (<= 0: SM count x resident CTAs), `parity` the step's Ctrl slot.

@@ -72,17 +72,20 @@ static cudaError_t init_hancock() {
   return e;
 }
 
-static cudaError_t init() {
-  cudaError_t e;
-  if ((e = init_pol<PolF64>()) != cudaSuccess) return e;
-  if ((e = init_pol<PolF32>()) != cudaSuccess) return e;
-  if ((e = init_hancock<PolF64, true>()) != cudaSuccess) return e;
-  if ((e = init_hancock<PolF64, false>()) != cudaSuccess) return e;
-  if ((e = init_hancock<PolF32, true>()) != cudaSuccess) return e;
-  if ((e = init_hancock<PolF32, false>()) != cudaSuccess) return e;
-  if ((e = init_hancock<PolMixed, true>()) != cudaSuccess) return e;
-  if ((e = init_hancock<PolMixed, false>()) != cudaSuccess) return e;
-  return init_pol<PolMixed>();
+template <class Pol>
+static cudaError_t init_precision() {
+  cudaError_t e = init_pol<Pol>();
+  if (e == cudaSuccess) e = init_hancock<Pol, true>();
+  return e == cudaSuccess ? init_hancock<Pol, false>() : e;
+}
+
+static cudaError_t init(int precision) {
+  switch (precision) {
+    case PREC_FP64: return init_precision<PolF64>();
+    case PREC_FP32: return init_precision<PolF32>();
+    case PREC_MIXED: return init_precision<PolMixed>();
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 static int sm_count() {

@@ -99,8 +99,9 @@ int setup_device(int dev, unsigned char** base) {
   if (!d.done) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || p == nullptr) return PMHD_ERR_CUDA;
-    if (kernel_table_exact().init() != cudaSuccess || kernel_table_fast().init() != cudaSuccess)
-      return PMHD_ERR_CUDA;
+    for (int prec = PREC_FP64; prec <= PREC_MIXED; prec++)
+      if (kernel_table_exact().init(prec) != cudaSuccess || kernel_table_fast().init(prec) != cudaSuccess)
+        return PMHD_ERR_CUDA;
     d.base = static_cast<unsigned char*>(p);
     d.done = true;
   }

@@ -34,7 +34,7 @@ using namespace pmhd;
 namespace {
 
 std::mutex g_init_mu;
-bool g_init_done[64][2];
+bool g_init_done[64][2][3];
 
 }  // namespace
 
@@ -224,12 +224,12 @@ int pmhd_create(const pmhd_config* cfg, pmhd_solver** out) {
   {
     std::lock_guard<std::mutex> lk(g_init_mu);
     const int dev = cfg->device & 63, which = cfg->exact ? 1 : 0;
-    if (!g_init_done[dev][which]) {
-      if (s->kt->init() != cudaSuccess) {
+    if (!g_init_done[dev][which][cfg->precision]) {
+      if (s->kt->init(cfg->precision) != cudaSuccess) {
         delete s;
         return PMHD_ERR_CUDA;
       }
-      g_init_done[dev][which] = true;
+      g_init_done[dev][which][cfg->precision] = true;
     }
   }
   s->elem = cfg->precision == PMHD_FP32 ? 4 : 8;
