@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 
 #include "learned/conv.h"
 #include "learned/net.h"
@@ -11,36 +12,47 @@
 
 namespace {
 
-__device__ int g_conv_err;  // set by a kernel whose bounded wait expired
+// Error word of the calling thread's convolution calls: pinned host memory the
+// kernels write directly when a bounded wait expires, so a call needs no clearing
+// and no copy on the stream -- one launch and one synchronisation.  Every thread
+// has its own (calls are synchronous), freed when the thread ends.
+struct ErrorWord {
+  int* p = nullptr;
+  ~ErrorWord() {
+    if (p) cudaFreeHost(p);
+  }
+};
 
-// Device address of the error word; the first call on a device also sets the
+// The thread's error word, cleared; the first call on a device also sets the
 // kernels' shared-memory limits there.
 int* error_word() {
-  static int prepared_dev = -1;
+  static std::mutex mu;
+  static bool prepared[64];
+  static thread_local ErrorWord word;
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  if (dev != prepared_dev) {
-    if (pmhd::learned::conv_prepare() != cudaSuccess) return nullptr;
-    prepared_dev = dev;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!prepared[dev]) {
+      if (pmhd::learned::conv_prepare() != cudaSuccess) return nullptr;
+      prepared[dev] = true;
+    }
   }
-  int* p = nullptr;
-  if (cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_conv_err) != cudaSuccess) return nullptr;
-  return p;
+  if (!word.p && cudaHostAlloc(&word.p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
+    return nullptr;
+  *word.p = 0;
+  return word.p;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-int finish(cudaError_t e, int* err, cudaStream_t s) {
+int finish(cudaError_t e, const int* err, cudaStream_t s) {
   if (e == cudaErrorNotSupported) return PMHD_ERR_UNSUPPORTED;
   if (e != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
     cudaGetLastError();
     return PMHD_ERR_CUDA;
   }
-  int h = 0;
-  if (cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess)
-    return PMHD_ERR_CUDA;
-  return h ? PMHD_ERR_TIMEOUT : PMHD_OK;
+  return *static_cast<const volatile int*>(err) ? PMHD_ERR_TIMEOUT : PMHD_OK;
 }
 
 }  // namespace
@@ -58,7 +70,6 @@ int pmhd_conv3x3(int mode, const void* x, int batch, int h, int w, int c_in, con
   int* err = error_word();
   if (!err) return PMHD_ERR_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return PMHD_ERR_CUDA;
   const cudaError_t e = pmhd::learned::conv3x3(mode, static_cast<const __nv_bfloat16*>(x), batch, h, w, c_in,
                                                static_cast<const __nv_bfloat16*>(weight), bias, c_out,
                                                static_cast<const __nv_bfloat16*>(z_prev), out0, out1, err, s);
@@ -72,7 +83,6 @@ int pmhd_conv3x3_wgrad(const void* x, const void* dz, int batch, int h, int w, i
   int* err = error_word();
   if (!err) return PMHD_ERR_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return PMHD_ERR_CUDA;
   const cudaError_t e = pmhd::learned::conv3x3_wgrad(static_cast<const __nv_bfloat16*>(x),
                                                      static_cast<const __nv_bfloat16*>(dz), batch, h, w, c_in, c_out,
                                                      dweight, dbias, err, s);

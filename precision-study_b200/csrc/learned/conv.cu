@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
       if (lane == 0) mbar_arrive(tempty + b);
     }
   }
-  if (!ok && lane == 0) atomicExch(err, PMHD_LEARNED_ERR_TIMEOUT);
+  if (!ok && lane == 0) *static_cast<volatile int*>(err) = PMHD_LEARNED_ERR_TIMEOUT;
   umma::fence_before_sync();
   __syncthreads();
   if (warp == 0) {
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __nv_bfloat1
       }
     }
   }
-  if (!ok && lane == 0) atomicExch(err, PMHD_LEARNED_ERR_TIMEOUT);
+  if (!ok && lane == 0) *static_cast<volatile int*>(err) = PMHD_LEARNED_ERR_TIMEOUT;
   umma::fence_before_sync();
   __syncthreads();
   if (warp == 0) {

@@ -22,8 +22,8 @@ cudaError_t conv_prepare();
 //                the layer's weight transposed to [c_out][9][c_in] with c_in
 //                = the layer's outputs
 // Supported (c_in, c_out): GELU (32, 32); LINEAR (32, 16); DGELU (16, 32),
-// (32, 32).  cudaErrorNotSupported otherwise.  *err is set (non-zero) when
-// a bounded wait of the kernel expired.
+// (32, 32).  cudaErrorNotSupported otherwise.  *err (device or mapped host
+// memory) is set to non-zero when a bounded wait of the kernel expired.
 cudaError_t conv3x3(int mode, const __nv_bfloat16* x, int batch, int h, int w, int c_in, const __nv_bfloat16* wt,
                     const float* bias, int c_out, const __nv_bfloat16* zprev, void* out0, void* out1, int* err,
                     cudaStream_t s);
