@@ -64,19 +64,25 @@ __device__ __forceinline__ double fast_rsqrt(double x) {
   const double e = fma(-(x * y), y, 1.0);
   return fma(y, e * fma(e, 0.375, 0.5), y);
 }
-__device__ __forceinline__ double fast_sqrt(double x) {
+// Root of a positive normal number (no zero, infinity or NaN to look after).
+__device__ __forceinline__ double fast_sqrt_pos(double x) {
   const double y = rsqrt_seed(x);
   const double h = x * y;
   const double e = fma(-h, y, 1.0);
   const double s = fma(h, e * fma(e, 0.375, 0.5), h);
-  const double s1 = fma(fma(-s, s, x), 0.5 * y, s);
-  return x + x == x ? x : s1;
+  return fma(fma(-s, s, x), 0.5 * y, s);
+}
+__device__ __forceinline__ double fast_sqrt(double x) {
+  const double s = fast_sqrt_pos(x);
+  return x + x == x ? x : s;
 }
 #else
 inline double fast_rcp(double x) { return 1.0 / x; }
 inline double fast_rsqrt(double x) { return 1.0 / std::sqrt(x); }
 inline double fast_sqrt(double x) { return std::sqrt(x); }
+inline double fast_sqrt_pos(double x) { return std::sqrt(x); }
 #endif
+PMHD_HD float fast_sqrt_pos(float x) { return fast_sqrt(x); }
 
 }  // namespace pmhd
 

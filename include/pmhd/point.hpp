@@ -947,8 +947,10 @@ PMHD_HD T face_cf(T p, T inv, T bn2, T bt2s, const Phys<T>& ph) {
   const T a2 = ph.gamma * at_least(p, p_floor<T>()) * inv;
   const T can2 = bn2 * inv;
   const T sum = a2 + (can2 + bt2s * inv);
-  const T disc = at_least(sum * sum - (T)4.0 * a2 * can2, (T)0.0);
-  return fast_sqrt((T)0.5 * (sum + fast_sqrt(disc)));
+  // a2 > 0, so sum is positive; a discriminant of zero (or rounded below it)
+  // becomes 1e-300, whose root vanishes beside sum.
+  const T disc = at_least(sum * sum - (T)4.0 * a2 * can2, (T)1.0e-300);
+  return fast_sqrt_pos((T)0.5 * (sum + fast_sqrt_pos(disc)));
 }
 
 // Side of a face given by its primitives, B_n := bn.
@@ -1212,7 +1214,11 @@ PMHD_HD T cell_speed_fast(const T* P, const Phys<T>& ph) {
 PMHD_HD float minmod_fast(float a, float b) { return vmax(vmin(a, b), vmin(vmax(a, b), 0.0f)); }
 PMHD_HD double minmod_fast(double a, double b) {
   const double m = vabs(a) < vabs(b) ? a : b;
+#if defined(__CUDA_ARCH__)
+  return (__double2hiint(a) ^ __double2hiint(b)) < 0 ? 0.0 : m;  // signs differ (m is 0 if either is)
+#else
   return a * b > 0.0 ? m : 0.0;
+#endif
 }
 
 }  // namespace pmhd
