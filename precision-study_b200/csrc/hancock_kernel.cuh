@@ -25,11 +25,18 @@
 // so the interface fluxes reuse their storage.  Binary64 faces use 32 x 4
 // tiles: with 32 x 8 the tile needs ~200 KB and one CTA of 8 warps per SM
 // (latency-bound); at 32 x 4 two CTAs fit (98 KB; binary32 faces: 98 KB or
-// 82 KB at 32 x 8).  Registers are sized for two CTAs (128 per thread).
+// 82 KB at 32 x 8).  Registers are sized for two CTAs (128 per thread; 96 for the
+// ten warps of the performance build's binary64, which with glm_flux_lean and the
+// lean faces takes 77 us a step at 512^2 and 1.15 ms at 2048^2, against 106 / 1.66
+// with eight warps, two rounds of flux items and four faces in registers; 32 x 7
+// tiles of 512 threads, one CTA: 76 us / 1.18 ms).
 template <class S, class R>
 struct HancockTile {
   static constexpr int TYH = sizeof(R) == 8 ? 4 : 8;
   static constexpr int MINB = 2;                   // resident CTAs the registers are sized for
+  // Threads: the performance build's binary64 has a warp for each of the ten rows
+  // of interfaces (hancock_fluxes_lean), at 96 registers.
+  static constexpr int NT = kLeanFlux<R> ? 320 : 256;
   static constexpr int RW = TX + 4, RH = TYH + 4;  // region 36 x (TYH + 4)
   static constexpr int NR = RW * RH;
   static constexpr int BW = TX + 2, BH = TYH + 2;  // evolved-face box 34 x (TYH + 2)
@@ -86,14 +93,21 @@ struct HancockScalars {
   }
 };
 
+template <int AX>
+struct AxisTag {
+  static constexpr int value = AX;
+};
+
 // Primitives of region cells first, first + step, ... from the region's
 // conserved states in shared memory, in the storage precision (the mixed
-// policy's binary64 recovery), kept in the face precision.
+// policy's binary64 recovery), kept in the face precision.  Returns whether this
+// thread's cells are all usable (cell_usable_fast; kLeanFlux policies only).
 template <class Pol>
-__device__ __forceinline__ void hancock_recover(HancockTileOf<Pol>& s, const Phys<typename Pol::S>& phS, int first,
+__device__ __forceinline__ bool hancock_recover(HancockTileOf<Pol>& s, const Phys<typename Pol::S>& phS, int first,
                                                 int step) {
   using S = typename Pol::S;
   using R = typename Pol::R;
+  bool usable = true;
   for (int q = first; q < HancockTileOf<Pol>::NR; q += step) {
     S U9[NVAR], P9[NVAR];
 #pragma unroll
@@ -101,6 +115,88 @@ __device__ __forceinline__ void hancock_recover(HancockTileOf<Pol>& s, const Phy
     recover_cell<Pol>(U9, P9, phS);
 #pragma unroll
     for (int k = 0; k < NVAR; k++) s.P[k][q] = (R)P9[k];
+    if constexpr (kLeanFlux<R>) usable = usable && cell_usable_fast<R>(P9);
+  }
+  return usable;
+}
+
+// hancock_faces for the performance build's binary64: the four faces leave as
+// conserved states through shared memory while their fluxes accumulate in the
+// correction, then evolve in place, so nine values of the correction and one face
+// are live instead of four faces and four fluxes.  The reconstruction tests its
+// faces only when a cell of the region is unusable (checks), energies multiply by
+// 1 / (gamma - 1).  (Before: 1,700 instructions a cell, two thirds of the step's.)
+template <class Pol>
+__device__ __forceinline__ void hancock_faces_lean(HancockTileOf<Pol>& s, const HancockScalars<Pol>& c0,
+                                                   const Phys<typename Pol::R>& ph, bool checks, int first, int step) {
+  using R = typename Pol::R;
+  using HT = HancockTileOf<Pol>;
+  constexpr int RW = HT::RW, BW = HT::BW, BH = HT::BH, NB = HT::NB;
+  const R ch2 = c0.ch * c0.ch;
+  for (int q = first; q < NB; q += step) {
+    const int br = q / BW, bc = q % BW;
+    if ((br == 0 || br == BH - 1) && (bc == 0 || bc == BW - 1)) continue;
+    const int c = (br + 1) * RW + (bc + 1);
+    R corr[NVAR];
+    auto direction = [&](auto axis) {
+      constexpr int AX = decltype(axis)::value;
+      const int d = AX ? RW : 1;
+      const R h = AX ? c0.hy : c0.hx;
+      bool ok = true;  // recon_cell's test of both faces
+      if (checks) {
+#pragma unroll
+        for (int k = 0; k < NVAR; k++) {
+          const R p0 = s.P[k][c], sl = (R)0.5 * minmod(p0 - s.P[k][c - d], s.P[k][c + d] - p0);
+          const R lo = p0 - sl, hi = p0 + sl;
+          if (k == RHO) ok = ok && !(lo <= rho_floor<R>()) && !(hi <= rho_floor<R>());
+          if (k == EN) ok = ok && !(lo <= p_floor<R>()) && !(hi <= p_floor<R>());
+          ok = ok && vfinite(lo) && vfinite(hi);
+        }
+      }
+      R P0[NVAR], sl[NVAR];
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) {
+        P0[k] = s.P[k][c];
+        const R a = P0[k] - s.P[k][c - d], b = s.P[k][c + d] - P0[k];
+        sl[k] = ok ? (R)0.5 * (checks ? minmod(a, b) : minmod_fast(a, b)) : (R)0;
+      }
+      R dF[NVAR];  // upper minus lower, one rounding: mirror images get mirrored values
+#pragma unroll
+      for (int side = 0; side < 2; side++) {
+        R P[NVAR], U[NVAR], F[NVAR];
+#pragma unroll
+        for (int k = 0; k < NVAR; k++) P[k] = side ? P0[k] + sl[k] : P0[k] - sl[k];
+        const R v2 = P[MX] * P[MX] + P[MY] * P[MY] + P[MZ] * P[MZ];
+        const R b2 = P[BX] * P[BX] + P[BY] * P[BY] + P[BZ] * P[BZ];
+        U[RHO] = P[RHO];
+        U[MX] = P[RHO] * P[MX];
+        U[MY] = P[RHO] * P[MY];
+        U[MZ] = P[RHO] * P[MZ];
+        U[EN] = P[EN] * ph.inv_gm1 + (R)0.5 * P[RHO] * v2 + (R)0.5 * b2;
+        U[BX] = P[BX], U[BY] = P[BY], U[BZ] = P[BZ], U[PSI] = P[PSI];
+        glm_phys_flux_prim<R, AX>(P, U[EN], ch2, F);
+#pragma unroll
+        for (int k = 0; k < NVAR; k++) {
+          s.H[2 * AX + side][k][q] = U[k];
+          dF[k] = side ? F[k] - dF[k] : F[k];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) corr[k] = AX ? corr[k] + h * dF[k] : h * dF[k];
+    };
+    direction(AxisTag<0>{});
+    direction(AxisTag<1>{});
+#pragma unroll 1
+    for (int f = 0; f < 4; f++) {
+      R h[NVAR];
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) h[k] = s.H[f][k][q] - corr[k];
+      h[PSI] = h[PSI] - c0.hdamp * s.H[f][PSI][q];
+      if (state_usable_fast<R>(h, ph)) {
+#pragma unroll
+        for (int k = 0; k < NVAR; k++) s.H[f][k][q] = h[k];
+      }
+    }
   }
 }
 
@@ -169,11 +265,6 @@ __device__ __forceinline__ void hancock_faces(HancockTileOf<Pol>& s, const Hanco
   }
 }
 
-template <int AX>
-struct AxisTag {
-  static constexpr int value = AX;
-};
-
 // Interface fluxes of the tile at (i0, j0): x-interface (r, c) = between
 // tile columns c-1 and c (c = 0..32) of tile row r; y-interface (r, c) =
 // between tile rows r-1 and r (r = 0..TYH) of tile column c.  Stored over
@@ -190,42 +281,30 @@ __device__ __forceinline__ void hancock_fluxes(HancockTileOf<Pol>& s, const Memb
   R* Gy = &s.f.Gy[0][0];
   const GlmK<R> gk = GlmK<R>::make(ch);
   for (int q = first; q < HT::NFX + HT::NGY; q += step) {
+    R a[NVAR], b[NVAR], F[NVAR];
     int st;
-    auto flux = [&](auto axis, const R* ha, const R* hb, R* out, int n_out) {  // faces at ha / hb, plane stride NB
-      constexpr int AX = decltype(axis)::value;
-      if constexpr (kLeanFlux<R>) {
-        return glm_flux_lean<R, AX, true>(
-            gk, HLLD, ph,
-            [&](R* a, R* b) {
-#pragma unroll
-              for (int k = 0; k < NVAR; k++) {
-                a[k] = ha[k * HT::NB];
-                b[k] = hb[k * HT::NB];
-              }
-            },
-            [&](int k, R f) { out[k * n_out] = f; });
-      } else {
-        R a[NVAR], b[NVAR], F[NVAR];
-#pragma unroll
-        for (int k = 0; k < NVAR; k++) {
-          a[k] = ha[k * HT::NB];
-          b[k] = hb[k * HT::NB];
-        }
-        const int code = PMHD_FAST_FLUX ? glm_flux_fast_cons<R, AX>(a, b, gk, HLLD, F, ph)
-                                        : glm_flux<R, AX>(a, b, ch, HLLD, F, ph);
-#pragma unroll
-        for (int k = 0; k < NVAR; k++) out[k * n_out] = F[k];
-        return code;
-      }
-    };
     if (q < HT::NFX) {
       const int r = q / (TX + 1), c = q % (TX + 1);
       const int bl = (r + 1) * BW + c, br = bl + 1;  // box cells left / right of the interface
-      st = flux(AxisTag<0>{}, &s.H[1][0][bl], &s.H[0][0][br], Fx + q, HT::NFX);
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) {
+        a[k] = s.H[1][k][bl];
+        b[k] = s.H[0][k][br];
+      }
+      st = PMHD_FAST_FLUX ? glm_flux_fast_cons<R, 0>(a, b, gk, HLLD, F, ph) : glm_flux<R, 0>(a, b, ch, HLLD, F, ph);
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) Fx[k * HT::NFX + q] = F[k];
     } else {
       const int g = q - HT::NFX, r = g / TX, c = g % TX;
       const int bb = r * BW + (c + 1), bt = bb + BW;  // box cells below / above
-      st = flux(AxisTag<1>{}, &s.H[3][0][bb], &s.H[2][0][bt], Gy + g, HT::NGY);
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) {
+        a[k] = s.H[3][k][bb];
+        b[k] = s.H[2][k][bt];
+      }
+      st = PMHD_FAST_FLUX ? glm_flux_fast_cons<R, 1>(a, b, gk, HLLD, F, ph) : glm_flux<R, 1>(a, b, ch, HLLD, F, ph);
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) Gy[k * HT::NGY + g] = F[k];
     }
     if (HLLD) {
       // Count each interface of the domain once: interface I (between
@@ -239,6 +318,51 @@ __device__ __forceinline__ void hancock_fluxes(HancockTileOf<Pol>& s, const Memb
         const int g = q - HT::NFX, r = g / TX, c = g % TX, J = j0 + r;
         inside = i0 + c < m.nx && J <= m.ny && (r < TYH || J == m.ny);
       }
+      if (inside) {
+        n_deg += st == HLLD_FALLBACK_DEGENERATE ? 1u : 0u;
+        n_np += st == HLLD_FALLBACK_NONPHYSICAL ? 1u : 0u;
+      }
+    }
+  }
+}
+
+// hancock_fluxes for the performance build's binary64 (glm_flux_lean): a warp's 32
+// items are one row of x-interfaces (right of a row's cells), one row of
+// y-interfaces, or the tile's left column, through one copy of the flux code in
+// x-normal order (slots exchanged for y, as face_flux does).
+template <class Pol, bool HLLD>
+__device__ __forceinline__ void hancock_fluxes_lean(HancockTileOf<Pol>& s, const Member& m, int i0, int j0,
+                                                    typename Pol::R ch, const Phys<typename Pol::R>& ph, int first,
+                                                    int step, unsigned& n_deg, unsigned& n_np) {
+  using R = typename Pol::R;
+  using HT = HancockTileOf<Pol>;
+  constexpr int BW = HT::BW, TYH = HT::TYH, NB = HT::NB;
+  const GlmK<R> gk = GlmK<R>::make(ch);
+#pragma unroll 1
+  for (int q = first; q < (2 * TYH + 2) * 32; q += step) {
+    const int u = q >> 5, lane = q & 31;
+    const bool axis = u >= TYH && u <= 2 * TYH;
+    const int r = axis ? u - TYH : (u < TYH ? u : lane), c = axis ? lane : (u < TYH ? lane + 1 : 0);
+    if (u == 2 * TYH + 1 && lane >= TYH) continue;
+    // Box cells below / above (y) or left / right (x) of the interface.
+    const R* ha = axis ? &s.H[3][0][r * BW + c + 1] : &s.H[1][0][(r + 1) * BW + c];
+    const R* hb = axis ? &s.H[2][0][(r + 1) * BW + c + 1] : &s.H[0][0][(r + 1) * BW + c + 1];
+    R* out = axis ? &s.f.Gy[0][r * TX + c] : &s.f.Fx[0][r * (TX + 1) + c];
+    const int n_out = axis ? HT::NGY : HT::NFX;
+    const int s1 = axis ? 2 : 1, s2 = axis ? 1 : 2, s5 = axis ? 6 : 5, s6 = axis ? 5 : 6;
+    auto slot = [&](int k) { return k == 1 ? s1 : k == 2 ? s2 : k == 5 ? s5 : k == 6 ? s6 : k; };
+    auto load = [&](R* a, R* b) {
+#pragma unroll
+      for (int k = 0; k < NVAR; k++) {
+        a[k] = ha[slot(k) * NB];
+        b[k] = hb[slot(k) * NB];
+      }
+    };
+    const int st = glm_flux_lean<R, 0, true>(gk, HLLD, ph, load, [&](int k, R f) { out[slot(k) * n_out] = f; });
+    if (HLLD) {  // each interface of the domain once (see hancock_fluxes)
+      const int I = i0 + c, J = j0 + r;
+      const bool inside = axis ? I < m.nx && J <= m.ny && (r < TYH || J == m.ny)
+                               : J < m.ny && I <= m.nx && (c < TX || I == m.nx);
       if (inside) {
         n_deg += st == HLLD_FALLBACK_DEGENERATE ? 1u : 0u;
         n_np += st == HLLD_FALLBACK_NONPHYSICAL ? 1u : 0u;
@@ -350,7 +474,7 @@ __device__ __forceinline__ void hancock_flush(const Member& m, int p, int lane, 
 // One CTA per tile, plain coalesced loads (the binary64 policy, whose 32 x 4
 // tiles have no TMA descriptor).
 template <class Pol, bool HLLD>
-__global__ void __launch_bounds__(256, HancockTileOf<Pol>::MINB) hancock_kernel(const __grid_constant__ Member m, const int p) {
+__global__ void __launch_bounds__(HancockTileOf<Pol>::NT, HancockTileOf<Pol>::MINB) hancock_kernel(const __grid_constant__ Member m, const int p) {
   using S = typename Pol::S;
   using R = typename Pol::R;
   using HT = HancockTileOf<Pol>;
@@ -379,13 +503,19 @@ __global__ void __launch_bounds__(256, HancockTileOf<Pol>::MINB) hancock_kernel(
 #pragma unroll
     for (int k = 0; k < NVAR; k++) s.U[k][q] = uin[(size_t)k * m.plane + (size_t)gj * m.pitch + gi];
   }
-  hancock_recover<Pol>(s, phS, tid, blockDim.x);  // each thread recovers the cells it loaded
-  __syncthreads();
+  // Each thread recovers the cells it loaded.
+  const bool all_usable = __syncthreads_and(hancock_recover<Pol>(s, phS, tid, blockDim.x));
   const HancockScalars<Pol> c0(m, v);
-  hancock_faces<Pol>(s, c0, ph, tid, blockDim.x);
+  if constexpr (kLeanFlux<R>)
+    hancock_faces_lean<Pol>(s, c0, ph, !all_usable, tid, blockDim.x);
+  else
+    hancock_faces<Pol>(s, c0, ph, tid, blockDim.x);
   __syncthreads();
   unsigned n_deg = 0, n_np = 0;
-  hancock_fluxes<Pol, HLLD>(s, m, i0, j0, c0.ch, ph, tid, blockDim.x, n_deg, n_np);
+  if constexpr (kLeanFlux<R>)
+    hancock_fluxes_lean<Pol, HLLD>(s, m, i0, j0, c0.ch, ph, tid, blockDim.x, n_deg, n_np);
+  else
+    hancock_fluxes<Pol, HLLD>(s, m, i0, j0, c0.ch, ph, tid, blockDim.x, n_deg, n_np);
   __syncthreads();
   unsigned long long sp = 0;
   hancock_update<Pol, true>(s, m, v, c0, uin, uout, i0, j0, phS, ph, tid, blockDim.x, sp);

@@ -323,9 +323,9 @@ static cudaError_t hancock_pol(int hlld, int part, const Member& m, int parity, 
       hancock_persistent_kernel<Pol, false><<<grid, 256, smem, s>>>(m, parity);
   } else {
     if (hlld)
-      hancock_kernel<Pol, true><<<ntiles, 256, smem, s>>>(m, parity);
+      hancock_kernel<Pol, true><<<ntiles, HancockTileOf<Pol>::NT, smem, s>>>(m, parity);
     else
-      hancock_kernel<Pol, false><<<ntiles, 256, smem, s>>>(m, parity);
+      hancock_kernel<Pol, false><<<ntiles, HancockTileOf<Pol>::NT, smem, s>>>(m, parity);
   }
   return cudaGetLastError();
 }
