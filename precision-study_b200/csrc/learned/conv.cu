@@ -8,7 +8,7 @@
 //
 // Implicit GEMM.  Forward / backward-data: M = 128 output pixels x N = c_out
 // channels, K = 9 taps x c_in channels.  A persistent CTA per SM walks tiles of
-// 8 image rows x 128 pixels; a tile's input is staged once, each tap's operand
+// 8 (small images: 4 or 2) image rows x 128 pixels; a tile's input is staged once, each tap's operand
 // is a shifted descriptor into it, and producer, MMA and epilogue warps pipeline
 // the tiles.  Weight gradient: D[(row, c_in)][(row, c_out)] = sum over pixels of
 // x(p + tap) dz(p)^T, K = pixels; both operands are channel-major (MN-major) as
@@ -157,10 +157,9 @@ __device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void* src, bool
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 constexpr int kRowPix = 128;               // output pixels of a row segment (M)
-constexpr int kRows = 8;                   // output rows per tile
 constexpr int kRowPitch = kRowPix + 2;     // staged pixels per input row
 
-// A row tile: image bb, output rows y0 .. y0 + kRows - 1, pixels x0 .. x0 + 127,
+// A row tile: image bb, output rows y0 .., pixels x0 ..,
 // of which `rows` rows and `pix` pixels lie in the image.
 struct RowTile {
   long long bb;
@@ -256,12 +255,12 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Forward / backward-data kernel, any image size: persistent CTAs, one per SM,
-// loop over row tiles.  A tile is 8 image rows x 128 pixels; its 10 x 130 input
-// pixels (periodic) are staged once as NHWC has them (umma.cuh: a swizzled K-major
+// loop over row tiles.  A tile is ROWS (8, 4 or 2) image rows x 128 pixels; its
+// (ROWS + 2) x 130 input pixels (periodic) are staged once as NHWC has them (umma.cuh: a swizzled K-major
 // M = 128 operand whose rows are pixels), so the nine taps need no copies
 // (issue_row_mmas).  Five producer warps stage tile k + 1
 // while one thread issues tile k's MMAs and sixteen warps drain tile k - 1 from
-// tensor memory (128 lanes x CO columns per row, eight rows side by side); two
+// tensor memory (128 lanes x CO columns per row, the rows side by side); two
 // staging and two accumulator buffers, hand-offs by mbarriers:
 //   full[b]   producers -> MMA      staging buffer b holds its tile
 //   empty[b]  MMA commit -> producers  the MMAs that read buffer b are done
@@ -269,7 +268,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
 //   tempty[b] epilogue -> MMA          accumulator buffer b has been read
 // Every wait is bounded; on expiry the CTA records the error and leaves.
 // One 32 -> 32 GELU layer over 8 x 512^2 moves 403 MB (62 us at the 6.45 TB/s copy
-// rate): 111 us a call, about 75 of them the kernel's, against 174 before the
+// rate): 100 us a call, about 75 of them the kernel's, against 174 before the
 // swizzled staging (full L2 sectors: 131 -> 114), the N = 3 CO MMAs, constant
 // descriptor steps and sixteen epilogue warps with 32-byte stores.  What is left
 // over the copy: the 16 special-function operations a clock of GELU (2.2 us of a
@@ -277,14 +276,14 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
 constexpr int kPipeEpiWarps = 16, kPipeProdWarps = 5;
 constexpr int kPipeThreads = 32 * (kPipeEpiWarps + kPipeProdWarps + 1);
 
-template <int CG, int CO>
+template <int CG, int CO, int ROWS>
 struct PipeSmem {
-  static constexpr uint32_t kStage = ((kRows + 2) * kRowPitch * 2u * CG + 1023u) & ~1023u;  // one staging buffer
+  static constexpr uint32_t kStage = ((ROWS + 2) * kRowPitch * 2u * CG + 1023u) & ~1023u;  // one staging buffer
   static constexpr uint32_t kOffB = 2u * kStage;
   static constexpr uint32_t kBytesB = (uint32_t)CO * 9u * CG * 2u;
   static constexpr uint32_t kOffBar = (kOffB + kBytesB + 7u) & ~7u;
-  static constexpr uint32_t kBytes = kOffBar + 8u * 8u + 16u;
-  static constexpr uint32_t kColsBuf = umma::tmem_cols(kRows * CO);
+  static constexpr uint32_t kBytes = kOffBar + 9u * 8u + 8u;
+  static constexpr uint32_t kColsBuf = umma::tmem_cols(ROWS * CO);
   static constexpr uint32_t kTmemCols = 2u * kColsBuf;
   // Shared memory requested per CTA: at least enough that no more CTAs fit
   // on an SM (228 KB) than its 512 tensor-memory columns hold.
@@ -297,7 +296,7 @@ struct PipeSmem {
 //      CONV_LINEAR out0 = acc + bias (fp32)
 //      CONV_DGELU  out0 = acc * gelu'(zprev) (bf16); taps mirrored (the
 //                  transposed convolution of the backward pass)
-template <int CG, int CO, int EPI>
+template <int CG, int CO, int EPI, int ROWS>
 __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __nv_bfloat16* __restrict__ x,
                                                                        const __nv_bfloat16* __restrict__ wt,
                                                                        const float* __restrict__ bias,
@@ -306,14 +305,15 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
                                                                        void* __restrict__ out0,
                                                                        void* __restrict__ out1, int wide,
                                                                        int* __restrict__ err) {
-  using S = PipeSmem<CG, CO>;
+  using S = PipeSmem<CG, CO, ROWS>;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* sB = smem + S::kOffB;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::kOffBar);
   uint64_t* empty = full + 2;
   uint64_t* tfull = full + 4;
   uint64_t* tempty = full + 6;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(full + 8);
+  uint64_t* wfull = full + 8;  // epilogue warps -> MMA: weights and bias are staged
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(full + 9);
   __shared__ __align__(16) float sbias[CO];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -328,11 +328,9 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
       mbar_init(tfull + b, 1);
       mbar_init(tempty + b, kPipeEpiWarps);
     }
+    mbar_init(wfull, kPipeEpiWarps * 32);
     fence_barrier_init();
   }
-  if (tid < CO) sbias[tid] = EPI == CONV_DGELU ? 0.0f : bias[tid];
-  stage_weights<CG, CO, EPI>(sB, wt, tid, kPipeThreads);
-  fence_proxy_async_smem();
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
@@ -350,9 +348,9 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
         ok = false;
         break;
       }
-      const RowTile rt = row_tile<kRows, kRowPix>(tile, h, w);
+      const RowTile rt = row_tile<ROWS, kRowPix>(tile, h, w);
       const uint32_t dst = smem_u32(smem + b * S::kStage);
-      for (int r = pw; r < kRows + 2; r += kPipeProdWarps)
+      for (int r = pw; r < ROWS + 2; r += kPipeProdWarps)
         stage_halo_row<CG, kRowPix, false>(dst + r * kRowPitch * 2 * CG, x, rt, r, h, w, lane);
       cp_wait_all();
       fence_proxy_async_smem();
@@ -362,9 +360,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
     // MMA issuer: tile k from buffer k % 2 into accumulator buffer k % 2
     // once the epilogue has read that buffer's previous tile (k - 2).
     int k = 0;
+    ok = warp_wait(wfull, 0);
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
       const int b = k & 1;
-      if (!warp_wait(full + b, (uint32_t)(k >> 1) & 1u) ||
+      if (!ok || !warp_wait(full + b, (uint32_t)(k >> 1) & 1u) ||
           (k >= 2 && !warp_wait(tempty + b, (uint32_t)((k >> 1) - 1) & 1u))) {
         ok = false;
         break;
@@ -372,7 +371,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
       umma::fence_after_sync();
       if (lane == 0) {
         issue_row_mmas<CG, CO>(smem_u32(smem + b * S::kStage), smem_u32(sB), tmem + (uint32_t)b * S::kColsBuf,
-                                    row_tile<kRows, kRowPix>(tile, h, w).rows);
+                                    row_tile<ROWS, kRowPix>(tile, h, w).rows);
         umma::commit(tfull + b);
         umma::commit(empty + b);
       }
@@ -384,7 +383,13 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
       if (kk >= 0 && !warp_wait(empty + (kk & 1), (uint32_t)(kk >> 1) & 1u)) ok = false;
   } else {
     // Epilogue warps: tile k from accumulator buffer k % 2; warp q + 4 r owns
-    // lane quarter q (pixels 32 q .. 32 q + 31) of rows r and r + 4.
+    // lane quarter q (pixels 32 q .. 32 q + 31) of rows r, r + 4, ...  First they
+    // stage the weights, while the producers load the first tile.
+    if (tid < CO) sbias[tid] = EPI == CONV_DGELU ? 0.0f : bias[tid];
+    stage_weights<CG, CO, EPI>(sB, wt, tid, kPipeEpiWarps * 32);
+    fence_proxy_async_smem();
+    mbar_arrive(wfull);
+    asm volatile("bar.sync 1, %0;" ::"n"(kPipeEpiWarps * 32) : "memory");  // sbias
     const int q = warp & 3;
     int k = 0;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
@@ -394,7 +399,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
         break;
       }
       umma::fence_after_sync();
-      const RowTile rt = row_tile<kRows, kRowPix>(tile, h, w);
+      const RowTile rt = row_tile<ROWS, kRowPix>(tile, h, w);
       if (q * 32 < rt.pix) {
         const bool in = q * 32 + lane < rt.pix;
 #pragma unroll 1
@@ -628,9 +633,22 @@ cudaError_t set_smem(K kernel, uint32_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+template <int CG, int CO, int EPI>
+cudaError_t prepare_conv() {
+  cudaError_t e = set_smem(conv3x3_pipe_kernel<CG, CO, EPI, 2>, PipeSmem<CG, CO, 2>::kLaunchBytes);
+  if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<CG, CO, EPI, 4>, PipeSmem<CG, CO, 4>::kLaunchBytes);
+  if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<CG, CO, EPI, 8>, PipeSmem<CG, CO, 8>::kLaunchBytes);
+  return e;
+}
+
 int g_sms = 0;  // SM count of the device the kernels were prepared on
 
 bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
+
+// Tiles of `rows` image rows x 128 pixels.
+long long row_tiles(int batch, int h, int w, int rows) {
+  return (long long)batch * ((h + rows - 1) / rows) * ((w + kRowPix - 1) / kRowPix);
+}
 
 // Persistent CTAs: one per SM, at most one per tile.  Test hook:
 // PMHD_CONV_MAX_CTAS > 0 limits them, so small images still give each CTA several
@@ -644,14 +662,29 @@ unsigned persistent_grid(long long tiles) {
   return (unsigned)grid;
 }
 
+template <int CG, int CO, int EPI, int ROWS>
+cudaError_t launch_rows(const __nv_bfloat16* x, int batch, int h, int w, const __nv_bfloat16* wt, const float* bias,
+                        const __nv_bfloat16* zprev, void* out0, void* out1, int* err, cudaStream_t s) {
+  const long long tiles = row_tiles(batch, h, w, ROWS);
+  const int wide = aligned32(out0) && (EPI != CONV_GELU || aligned32(out1)) && (EPI != CONV_DGELU || aligned32(zprev));
+  conv3x3_pipe_kernel<CG, CO, EPI, ROWS>
+      <<<persistent_grid(tiles), kPipeThreads, PipeSmem<CG, CO, ROWS>::kLaunchBytes, s>>>(x, wt, bias, zprev, tiles, h,
+                                                                                         w, out0, out1, wide, err);
+  return cudaGetLastError();
+}
+
+// Rows per tile: the fewest of 2, 4, 8 that leave every tile an SM of its own (a
+// launch is then one tile's load, MMAs and drain in sequence: 8 x 64^2 GELU layer
+// 32.5 -> 29.4 us a call with tiles of 4), else 8 (fewest halo rows).
 template <int CG, int CO, int EPI>
 cudaError_t launch_conv(const __nv_bfloat16* x, int batch, int h, int w, const __nv_bfloat16* wt, const float* bias,
                         const __nv_bfloat16* zprev, void* out0, void* out1, int* err, cudaStream_t s) {
-  const long long tiles = (long long)batch * ((h + kRows - 1) / kRows) * ((w + kRowPix - 1) / kRowPix);
-  const int wide = aligned32(out0) && (EPI != CONV_GELU || aligned32(out1)) && (EPI != CONV_DGELU || aligned32(zprev));
-  conv3x3_pipe_kernel<CG, CO, EPI><<<persistent_grid(tiles), kPipeThreads, PipeSmem<CG, CO>::kLaunchBytes, s>>>(
-      x, wt, bias, zprev, tiles, h, w, out0, out1, wide, err);
-  return cudaGetLastError();
+  const int sms = g_sms > 0 ? g_sms : 148;
+  if (row_tiles(batch, h, w, 2) <= sms)
+    return launch_rows<CG, CO, EPI, 2>(x, batch, h, w, wt, bias, zprev, out0, out1, err, s);
+  if (row_tiles(batch, h, w, 4) <= sms)
+    return launch_rows<CG, CO, EPI, 4>(x, batch, h, w, wt, bias, zprev, out0, out1, err, s);
+  return launch_rows<CG, CO, EPI, 8>(x, batch, h, w, wt, bias, zprev, out0, out1, err, s);
 }
 
 template <int CO>
@@ -668,10 +701,10 @@ cudaError_t conv_prepare() {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<32, 32, CONV_GELU>, PipeSmem<32, 32>::kLaunchBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<32, 16, CONV_LINEAR>, PipeSmem<32, 16>::kLaunchBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<16, 32, CONV_DGELU>, PipeSmem<16, 32>::kLaunchBytes);
-  if (e == cudaSuccess) e = set_smem(conv3x3_pipe_kernel<32, 32, CONV_DGELU>, PipeSmem<32, 32>::kLaunchBytes);
+  if (e == cudaSuccess) e = prepare_conv<32, 32, CONV_GELU>();
+  if (e == cudaSuccess) e = prepare_conv<32, 16, CONV_LINEAR>();
+  if (e == cudaSuccess) e = prepare_conv<16, 32, CONV_DGELU>();
+  if (e == cudaSuccess) e = prepare_conv<32, 32, CONV_DGELU>();
   if (e == cudaSuccess) e = set_smem(wgrad_kernel<32>, WgradSmem<32>::kBytes);
   if (e == cudaSuccess) e = set_smem(wgrad_kernel<16>, WgradSmem<16>::kBytes);
   return e;

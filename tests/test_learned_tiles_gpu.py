@@ -1,6 +1,6 @@
 """The tiled convolution kernels (pmhd_conv3x3, pmhd_conv3x3_wgrad) at the
-edges of their tiles -- 8 x 128 pixels forward and backward, 8 x 64 for the
-weight gradient -- against the float64 oracle: small integers, so every product
+edges of their tiles -- 2, 4 or 8 x 128 pixels forward and backward, 8 x 64 for
+the weight gradient -- against the float64 oracle: small integers, so every product
 and partial sum is exact in the fp32 accumulators and the results are equal."""
 import ctypes
 
@@ -12,8 +12,9 @@ from test_learned_gpu import C, _bf, _conv, _ints, _wgrad
 pytestmark = pytest.mark.gpu
 
 # One pixel; one less than, at and one more than a tile in each direction;
-# narrower than a halo; several segments.
-SHAPES = [(1, 1, 1), (1, 2, 3), (2, 7, 63), (1, 9, 65), (1, 8, 127), (1, 15, 129), (1, 17, 64), (2, 8, 257)]
+# narrower than a halo; several segments; images that take tiles of 4 and 8 rows
+# (more than 148 of the next smaller ones).
+SHAPES = [(1, 1, 1), (1, 2, 3), (2, 7, 63), (1, 9, 65), (1, 8, 127), (1, 15, 129), (1, 17, 64), (2, 8, 257), (8, 39, 65), (20, 33, 20)]
 
 
 @pytest.mark.parametrize("max_ctas", [0, 2])
