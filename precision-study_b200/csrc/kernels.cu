@@ -109,14 +109,17 @@ static int occupancy() {
   return per_sm;
 }
 
-// Tiles per run of a batched launch of `ntiles` tiles on `grid` CTAs: the
-// longest run (fewest re-reads of member descriptors and control slots) whose
-// busiest CTA gets at most 1/16 more tiles than it would with runs of one.
-// Short work lists need short runs: 16 members of 64^2 .. 256^2 (700 tiles on
-// 148 CTAs) as runs of 16 keep 44 CTAs busy; long lists (the 512-member
-// benchmark ensemble, 73,000 tiles) keep runs of 16.
+// Tiles per run of a batched launch of `ntiles` tiles on `grid` CTAs.  A run
+// flushes a member's counts and reads the next one's descriptor and control slot,
+// so short lists are one run a CTA (16 members of 64^2 .. 256^2, 700 tiles on 148
+// CTAs: 113 us a step, 123 as runs of one, 324 as 44 runs of 16); longer ones take
+// the longest power of two whose busiest CTA gets at most 1/16 more tiles than it
+// would with runs of one (the 512-member benchmark ensemble, 73,000 tiles: 16; 48
+// members of 64^2 .. 512^2: 880 us with 4, 894 with 11, where full tiles gather in
+// some CTAs and the grids' short edge tiles in others).
 static int batch_run(int ntiles, int grid) {
   const long long even = ((long long)ntiles + grid - 1) / grid;
+  if (even <= kBatchRunMax) return even > 1 ? (int)even : 1;
   for (int run = kBatchRunMax; run > 1; run /= 2) {
     const long long units = ((long long)ntiles + run - 1) / run;
     const long long most = (units + grid - 1) / grid * run;
@@ -130,7 +133,7 @@ static cudaError_t launch_one(int stage, const Batch& b, const Member& m0, int p
                               cudaStream_t s) {
   const size_t smem = Smem<Pol, TY>::total;
   auto go = [&](auto* kernel) {
-    kernel<<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run);
+    kernel<<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run, ((1u << 28) + run - 1) / run);
     return cudaGetLastError();
   };
   if constexpr (kPartial<TY>) {

@@ -504,11 +504,12 @@ __device__ __forceinline__ bool member_active(const Member& m, int p) {
 // scalars are then constant-bank operands and its TMA descriptors live in
 // parameter space); `b` only supplies the tile count.  BATCHED = true: the
 // members of `b`, read from device memory per tile, handed out in runs of
-// `run` (a power of two) consecutive tiles.  PARTIAL = true: tiles cover b.rows
+// `run` (1 .. 16) consecutive tiles.  PARTIAL = true: tiles cover b.rows
 // rows of the shape's (a runtime height costs 2 % on large grids).
 template <class Pol, int STAGE, bool HLLD, int TY, bool BATCHED, bool PARTIAL>
 __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
-    stage_kernel(const __grid_constant__ Member m0, const Batch b, const int p, const int run) {
+    stage_kernel(const __grid_constant__ Member m0, const Batch b, const int p, const int run,
+                 const unsigned inv_run) {
   using S = typename Pol::S;
   using R = typename Pol::R;
   using G = Geo<TY>;
@@ -541,10 +542,13 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
   // a member, so its descriptor, control slot and step values are re-read
   // once per member run instead of once per tile, while members that stop
   // early still leave their tiles spread over all CTAs.
+  // (t + 1) / run through the host's inv_run = 2^28 / run rounded up: exact for a
+  // power of two, and below 2^24 tiles for the other lengths, which only lists of
+  // at most 16 tiles a CTA get.  (A division here cost 1 % on long lists.)
   auto first_tile = [&]() { return BATCHED ? (int)blockIdx.x * run : (int)blockIdx.x; };
   auto after = [&](int t) {
     if constexpr (BATCHED)
-      return ((t + 1) & (run - 1)) != 0 ? t + 1 : t + 1 + ((int)gridDim.x - 1) * run;
+      return t + 1 != (int)__umulhi((unsigned)(t + 1) << 4, inv_run) * run ? t + 1 : t + 1 + ((int)gridDim.x - 1) * run;
     else
       return t + (int)gridDim.x;
   };

@@ -367,3 +367,11 @@ def test_every_run_length_covers_the_work_list(pmhd_lib, count):
         for k in range(count):
             assert e.member_stats(k).steps == 3
             np.testing.assert_array_equal(e.get_state(k), ref[k % 3])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [297, 700, 1600, 2220])
+def test_one_run_of_any_length_per_cta_covers_the_work_list(pmhd_lib, count):
+    """Short work lists are one run a CTA, of 3, 5, 11 and 15 tiles here (148
+    SMs): every member gets the bits of its single-grid run."""
+    test_every_run_length_covers_the_work_list(pmhd_lib, count)
