@@ -93,14 +93,17 @@ typedef struct {
   int device;                       /* CUDA device ordinal                     */
   int steps_per_graph;              /* steps captured per CUDA graph, 0 = auto */
   int autotune;                     /* 1: the first pmhd_advance that runs at least
-                                       32 steps times every stage-kernel variant
+                                       32 steps times the stage-kernel variants
                                        (tile shape x resident CTAs per SM)
                                        on 2 live steps each and keeps the fastest
                                        (an ensemble: per grid size, see below);
                                        results do not depend on the variant (up
-                                       to rounding when exact is 0).
-                                       0: 32x19 tiles, of fewer rows on small
-                                       grids, all resident CTAs.               */
+                                       to rounding when exact is 0, where two
+                                       tuned runs may choose differently).
+                                       0: a choice by grid size alone: 32x19
+                                       tiles, of fewer rows on small grids, or
+                                       on small binary64 grids (exact 0) 32x8,
+                                       32x4 or 32x2, all resident CTAs.        */
 } pmhd_config;
 
 typedef struct {
@@ -189,7 +192,9 @@ int pmhd_write_dat(pmhd_solver* s, const char* path, const char* title);
  * file ("PMHDRST1", int32 nx, ny, precision, element bytes, double t, int64
  * steps, values); pmhd_read_restart loads one into a handle of the same grid
  * and precision (PMHD_ERR_ARG otherwise, PMHD_ERR_IO on a bad file).  A run
- * resumed from a restart gives the same bits as one that never stopped. */
+ * resumed from a restart on the same device model gives the same bits as one
+ * that never stopped, unless exact is 0 and autotune is 1: the resumed run times
+ * the variants again and may choose another, equal up to rounding. */
 int pmhd_write_restart(pmhd_solver* s, const char* path);
 int pmhd_read_restart(pmhd_solver* s, const char* path);
 

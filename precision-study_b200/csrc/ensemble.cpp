@@ -167,9 +167,9 @@ cudaError_t make_work_list(pmhd_ensemble* e, const std::vector<int>& ms, int t, 
 
 // The autotuner of an ensemble: every size class (members of one grid size)
 // is timed on its own -- two live steps of only that class's members per
-// kernel variant (tile height x resident CTAs per SM); the variants compute
-// identical results, so these are ordinary steps of those members -- and
-// keeps its fastest variant.  The classes that chose the same tile height
+// kernel variant (tile height x resident CTAs per SM); the variants' results are
+// equal (parity build) or equal up to rounding, so these are ordinary steps of
+// those members -- and keeps its fastest variant.  The classes that chose the same tile height
 // then share one work list, whose CTA count is that of its largest class by
 // cells; a step launches each such part's stage 1, then each part's stage 2.
 // Returns the fewest tuning steps any member took (for step budgets) and

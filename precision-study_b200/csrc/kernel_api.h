@@ -28,8 +28,7 @@ enum Precision : int { PREC_FP64 = 0, PREC_FP32 = 1, PREC_MIXED = 2 };
 // plus kSplit for the shapes whose x and y interfaces go to separate warps.
 // Index into Member::tm and the Batch tile tables; index 0 is the default.  Every
 // precision has the first kNumBatchShapes, which are also the ones batches
-// (ensembles) run; the performance build's binary64 and binary32 kernels have
-// them all (single grids).
+// (ensembles) run; the performance build's binary64 has them all (single grids).
 #ifndef PMHD_TY0
 #define PMHD_TY0 19
 #endif
@@ -92,9 +91,8 @@ struct KernelTable {
                             int pitch, const int bc[4], cudaStream_t s);
   cudaError_t (*soa_to_aos)(int precision, const void* u, long long plane, int nx, int ny, int pitch, int layout,
                             void* aos, cudaStream_t s);
-  // Whether single grids of a precision can run a tile shape, and the one they
-  // run by default (indices into kTileShapes).
-  bool (*has_shape)(int precision, int idx);
+  // The tile shape single grids of a precision run by default (index into
+  // kTileShapes).
   int (*default_shape)(int precision, int nx, int ny);
   // Cell rows per tile of shape idx for one or more grids (nx, ny) in a launch.
   int (*tile_rows)(int idx, const int (*sizes)[2], int n);

@@ -44,9 +44,9 @@ static cudaError_t init_pol_ty() {
   return e != cudaSuccess ? e : init_pol_ty_b<Pol, TY, true>();
 }
 
-// The policy has the shapes past kNumBatchShapes.
+// The policy has the shapes past kNumBatchShapes: the performance build's binary64.
 template <class Pol>
-constexpr bool kAllShapes = PMHD_FAST_FLUX != 0 && !Pol::kMixed;
+constexpr bool kAllShapes = PMHD_FAST_FLUX != 0 && !Pol::kMixed && sizeof(typename Pol::R) == 8;
 
 template <class Pol>
 static cudaError_t init_pol() {
@@ -253,11 +253,6 @@ static int tile_rows(int idx, const int (*sizes)[2], int n) {
   return height;
 }
 
-static bool has_shape(int precision, int idx) {
-  return idx >= 0 && (idx < kNumBatchShapes || (idx < kNumTileShapes && PMHD_FAST_FLUX &&
-                                                (precision == PREC_FP64 || precision == PREC_FP32)));
-}
-
 static int grid_for(long long n) {
   long long b = (n + NTA - 1) / NTA;
   if (b > 148 * 64) b = 148 * 64;
@@ -360,9 +355,8 @@ const KernelTable& PMHD_TABLE_FN(PMHD_KNS)() {
   static const KernelTable t = {PMHD_STR(PMHD_KNS),          PMHD_KNS::init,
                                 PMHD_KNS::launch_stage,      PMHD_KNS::ctas_per_sm,
                                 PMHD_KNS::launch_speed,      PMHD_KNS::launch_aos_to_soa,
-                                PMHD_KNS::launch_soa_to_aos, PMHD_KNS::has_shape,         PMHD_KNS::default_shape,
-                                PMHD_KNS::tile_rows,
-                                PMHD_KNS::launch_hancock};
+                                PMHD_KNS::launch_soa_to_aos, PMHD_KNS::default_shape,
+                                PMHD_KNS::tile_rows,         PMHD_KNS::launch_hancock};
   return t;
 }
 

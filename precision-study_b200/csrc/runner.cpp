@@ -68,7 +68,9 @@ cudaError_t Runner::tune(int steps, TuneResult* res) {
   int ncand = 0;
   cudaError_t err = cudaSuccess;
   for (int ty = 0; ty < kNumTileShapes && err == cudaSuccess; ty++) {
-    if (!kt->has_shape(precision, ty) || (!single && ty >= kNumBatchShapes)) continue;
+    // Split shapes win or lose by size, not by timing: they only run where they
+    // are the default.
+    if (ty >= kNumBatchShapes && ty != saved.ty_idx) continue;
     const int occ = kt->ctas_per_sm(precision, hlld, ty, single == nullptr);
     for (int k = occ; k >= 1 && err == cudaSuccess; k--) {
       choice.ty_idx = ty;
@@ -81,7 +83,7 @@ cudaError_t Runner::tune(int steps, TuneResult* res) {
       cudaEventElapsedTime(&ms, e0, e1);
       ms /= (float)steps;
       ncand++;
-      if (ty == 0 && k == occ) default_ms = ms;
+      if (ty == saved.ty_idx && choice.grid == saved.grid) default_ms = ms;
       if (best_ms < 0.f || ms < best_ms) {
         best_ms = ms;
         best = choice;

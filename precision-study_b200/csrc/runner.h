@@ -23,7 +23,7 @@ struct TuneResult {
   LaunchChoice best;
   int candidates = 0;
   float best_ms_per_step = 0.f;
-  float default_ms_per_step = 0.f;  // the untuned choice (32 x 8, full occupancy)
+  float default_ms_per_step = 0.f;  // the untuned choice
 };
 
 // One work list of a multi-part launch plan (an ensemble whose size classes
@@ -60,10 +60,11 @@ class Runner {
   cudaError_t enqueue_steps(int nsteps) const;
   // Cached CUDA graph of `nsteps` steps for the current choice.
   int graph(int nsteps, cudaGraphExec_t* out);
-  // Times every variant (tile height x CTAs per SM) on `steps` live steps
-  // each (an even number), keeps the fastest in `choice`.  The variants
-  // compute identical results, so the timed steps are ordinary steps of the
-  // run.  Returns cudaSuccess or the first CUDA error.
+  // Times the variants (the batch shapes and the default one x CTAs per SM) on
+  // `steps` live steps each (an even number), keeps the fastest in `choice`.
+  // The variants' results are equal (parity build) or equal up to rounding, so
+  // the timed steps are ordinary steps of the run.  Returns cudaSuccess or the
+  // first CUDA error.
   cudaError_t tune(int steps, TuneResult* res);
   void release();
 

@@ -407,7 +407,8 @@ int pmhd_advance(pmhd_solver* s, double t_end, long long max_steps, pmhd_stats* 
   const int big = s->cfg.steps_per_graph;
   long long tune_steps = 0;
   if (s->cfg.autotune && !s->run.hancock && !s->tuned && (max_steps < 0 || max_steps >= 32)) {
-    // Live steps timed per kernel variant; identical results for every variant.
+    // Live steps timed per kernel variant (results equal, or equal up to rounding:
+    // Runner::tune).
     const int per = 2;
     PMHD_CU(s->run.tune(per, &s->tune_result));
     tune_steps = (long long)per * s->tune_result.candidates;
