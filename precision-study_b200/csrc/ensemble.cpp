@@ -204,7 +204,8 @@ cudaError_t tune_by_size(pmhd_ensemble* e, long long* min_steps, long long* laun
       LaunchPart part;
       part.ty_idx = t;
       int *dt = nullptr, *d0 = nullptr;
-      err = make_work_list(e, classes[c], t, &part.batch, &dt, &d0);
+      err = e->kt->init_stage(e->cfg.precision, e->run.hlld, t, 1);
+      if (err == cudaSuccess) err = make_work_list(e, classes[c], t, &part.batch, &dt, &d0);
       const int occ = e->kt->ctas_per_sm(e->cfg.precision, e->run.hlld, t, 1);
       for (int k = occ; k >= 1 && err == cudaSuccess; k--) {
         part.grid = k == occ ? 0 : sms * k;
@@ -372,7 +373,8 @@ int pmhd_ensemble_create(const pmhd_config* common, const pmhd_member_desc* memb
   e->failed.assign(n, 0);
   e->member_ty.assign(n, 0);
   int rc = PMHD_OK;
-  if (e->kt->init(common->precision) != cudaSuccess) rc = PMHD_ERR_CUDA;
+  const int hlld = common->solver == PMHD_SOLVER_HLLD ? 1 : 0;
+  if (e->kt->init_stage(common->precision, hlld, e->run.choice.ty_idx, 1) != cudaSuccess) rc = PMHD_ERR_CUDA;
   // Layout of the member states.
   e->hm.assign(n, Member());
   e->state_off.assign(n, 0);
@@ -410,7 +412,7 @@ int pmhd_ensemble_create(const pmhd_config* common, const pmhd_member_desc* memb
     m.ctrl = e->dCtrl + k;
     set_member_physics(m, d.x_min, d.x_max, d.y_min, d.y_max, d.gamma, common->hlld_tol, common->cfl, common->alpha,
                        common->order == PMHD_ORDER_MUSCL ? 1 : 0, d.bc, common->precision == PMHD_FP32);
-    if (!encode_member_tmaps(m, e->elem)) rc = PMHD_ERR_CUDA;
+    if (!encode_member_tmaps(m, e->elem, kNumBatchShapes)) rc = PMHD_ERR_CUDA;
   }
   if (rc == PMHD_OK &&
       cudaMemcpyAsync(e->dMembers, e->hm.data(), sizeof(Member) * n, cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
@@ -454,7 +456,7 @@ int pmhd_ensemble_create(const pmhd_config* common, const pmhd_member_desc* memb
   }
   e->run.kt = e->kt;
   e->run.precision = common->precision;
-  e->run.hlld = common->solver == PMHD_SOLVER_HLLD ? 1 : 0;
+  e->run.hlld = hlld;
   e->run.stream = e->stream;
   e->run.single = nullptr;
   // Initial states: built on the host, uploaded through the member's U1.

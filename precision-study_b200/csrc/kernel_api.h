@@ -71,9 +71,13 @@ struct Batch {
 
 struct KernelTable {
   const char* name;
-  // Sets the dynamic shared-memory limits of a precision's kernels (and so loads
-  // them); call once per process and device.
-  cudaError_t (*init)(int precision);
+  // Sets the dynamic shared-memory limits of the stage kernels of a tile shape (of
+  // the Hancock kernels), and so loads them: call on every device before the first
+  // launch or ctas_per_sm of that shape (loading all shapes at once made a
+  // process's first handle 40 ms instead of 28).  cudaErrorNotSupported: no such
+  // shape for the precision.
+  cudaError_t (*init_stage)(int precision, int hlld, int ty_idx, int batched);
+  cudaError_t (*init_hancock)(int precision, int hlld);
   // One SSPRK2 stage (1 or 2) over every member of the batch.  `ty_idx`
   // selects the tile shape (kTileShapes), `grid` the number of persistent
   // CTAs (<= 0: SM count x resident CTAs), `parity` the step's Ctrl slot.
@@ -105,10 +109,10 @@ struct KernelTable {
 const KernelTable& kernel_table_exact();
 const KernelTable& kernel_table_fast();
 
-// Fills the TMA descriptors of a member whose u, u1, plane, nx, ny and pitch
-// are set (member_setup.cpp).  Returns false if the driver entry point is
+// Fills the TMA descriptors of the first `shapes` tile shapes for a member whose
+// u, u1, plane, nx, ny and pitch are set (member_setup.cpp).  Returns false if the driver entry point is
 // missing or an encoding fails.
-bool encode_member_tmaps(Member& m, size_t elem_bytes);
+bool encode_member_tmaps(Member& m, size_t elem_bytes, int shapes);
 
 // Fills the time-type constants of a member from a configuration's physical
 // values, rounding to binary32 first when `fp32` (the reference's Real).

@@ -17,31 +17,31 @@ namespace PMHD_KNS {
 template <int TY>
 constexpr bool kPartial = TY == kTileShapes[0];
 
-template <class Pol, int STAGE, bool HLLD, int TY, bool BATCHED>
+using StageFn = void (*)(Member, Batch, int, int, unsigned);
+
+template <class Pol, bool HLLD, int TY, bool BATCHED>
+static StageFn stage_fn(int stage, bool partial) {
+  if constexpr (kPartial<TY>)
+    if (partial) return stage == 1 ? stage_kernel<Pol, 1, HLLD, TY, BATCHED, true> : stage_kernel<Pol, 2, HLLD, TY, BATCHED, true>;
+  return stage == 1 ? stage_kernel<Pol, 1, HLLD, TY, BATCHED, false> : stage_kernel<Pol, 2, HLLD, TY, BATCHED, false>;
+}
+
+template <class Pol, bool HLLD, int TY, bool BATCHED>
 static cudaError_t set_smem_attr() {
-  cudaError_t e = cudaFuncSetAttribute(stage_kernel<Pol, STAGE, HLLD, TY, BATCHED, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<Pol, TY>::total);
-  if constexpr (kPartial<TY>) {
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(stage_kernel<Pol, STAGE, HLLD, TY, BATCHED, true>,
+  cudaError_t e = cudaSuccess;
+  for (int partial = 0; partial <= (kPartial<TY> ? 1 : 0); partial++)
+    for (int stage = 1; stage <= 2 && e == cudaSuccess; stage++)
+      e = cudaFuncSetAttribute(stage_fn<Pol, HLLD, TY, BATCHED>(stage, partial != 0),
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<Pol, TY>::total);
-  }
   return e;
 }
 
-template <class Pol, int TY, bool BATCHED>
-static cudaError_t init_pol_ty_b() {
-  cudaError_t e;
-  if ((e = set_smem_attr<Pol, 1, true, TY, BATCHED>()) != cudaSuccess) return e;
-  if ((e = set_smem_attr<Pol, 2, true, TY, BATCHED>()) != cudaSuccess) return e;
-  if ((e = set_smem_attr<Pol, 1, false, TY, BATCHED>()) != cudaSuccess) return e;
-  return set_smem_attr<Pol, 2, false, TY, BATCHED>();
-}
-
-template <class Pol, int TY>
-static cudaError_t init_pol_ty() {
-  cudaError_t e = init_pol_ty_b<Pol, TY, false>();
-  return e != cudaSuccess ? e : init_pol_ty_b<Pol, TY, true>();
+template <class Pol, int TY, bool BATCHES>
+static cudaError_t init_pol_ty(int hlld, bool batched) {
+  if constexpr (BATCHES)
+    if (batched) return hlld ? set_smem_attr<Pol, true, TY, true>() : set_smem_attr<Pol, false, TY, true>();
+  if (batched) return cudaErrorNotSupported;
+  return hlld ? set_smem_attr<Pol, true, TY, false>() : set_smem_attr<Pol, false, TY, false>();
 }
 
 // The policy has the shapes past kNumBatchShapes: the performance build's binary64.
@@ -49,41 +49,40 @@ template <class Pol>
 constexpr bool kAllShapes = PMHD_FAST_FLUX != 0 && !Pol::kMixed && sizeof(typename Pol::R) == 8;
 
 template <class Pol>
-static cudaError_t init_pol() {
-  cudaError_t e;
-  if ((e = init_pol_ty<Pol, kTileShapes[0]>()) != cudaSuccess) return e;
+static cudaError_t init_pol(int hlld, int ty_idx, bool batched) {
+  if (ty_idx == 0) return init_pol_ty<Pol, kTileShapes[0], true>(hlld, batched);
+  if (ty_idx == 1) return init_pol_ty<Pol, kTileShapes[1], true>(hlld, batched);
   if constexpr (kAllShapes<Pol>) {
-    if ((e = init_pol_ty_b<Pol, kTileShapes[2], false>()) != cudaSuccess) return e;
-    if ((e = init_pol_ty_b<Pol, kTileShapes[3], false>()) != cudaSuccess) return e;
-    if ((e = init_pol_ty_b<Pol, kTileShapes[4], false>()) != cudaSuccess) return e;
+    if (ty_idx == 2) return init_pol_ty<Pol, kTileShapes[2], false>(hlld, batched);
+    if (ty_idx == 3) return init_pol_ty<Pol, kTileShapes[3], false>(hlld, batched);
+    if (ty_idx == 4) return init_pol_ty<Pol, kTileShapes[4], false>(hlld, batched);
   }
-  return init_pol_ty<Pol, kTileShapes[1]>();
+  return cudaErrorNotSupported;
+}
+
+static cudaError_t init_stage(int precision, int hlld, int ty_idx, int batched) {
+  switch (precision) {
+    case PREC_FP64: return init_pol<PolF64>(hlld, ty_idx, batched != 0);
+    case PREC_FP32: return init_pol<PolF32>(hlld, ty_idx, batched != 0);
+    case PREC_MIXED: return init_pol<PolMixed>(hlld, ty_idx, batched != 0);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 template <class Pol, bool HLLD>
-static cudaError_t init_hancock() {
+static cudaError_t init_hancock_pol() {
   const int smem = (int)sizeof(HancockTileOf<Pol>);
-  cudaError_t e = cudaFuncSetAttribute(hancock_kernel<Pol, HLLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if constexpr (HancockPersistent<Pol>::on) {
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(hancock_persistent_kernel<Pol, HLLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               smem);
-  }
-  return e;
+  if constexpr (HancockPersistent<Pol>::on)
+    return cudaFuncSetAttribute(hancock_persistent_kernel<Pol, HLLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  else
+    return cudaFuncSetAttribute(hancock_kernel<Pol, HLLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
-template <class Pol>
-static cudaError_t init_precision() {
-  cudaError_t e = init_pol<Pol>();
-  if (e == cudaSuccess) e = init_hancock<Pol, true>();
-  return e == cudaSuccess ? init_hancock<Pol, false>() : e;
-}
-
-static cudaError_t init(int precision) {
+static cudaError_t init_hancock(int precision, int hlld) {
   switch (precision) {
-    case PREC_FP64: return init_precision<PolF64>();
-    case PREC_FP32: return init_precision<PolF32>();
-    case PREC_MIXED: return init_precision<PolMixed>();
+    case PREC_FP64: return hlld ? init_hancock_pol<PolF64, true>() : init_hancock_pol<PolF64, false>();
+    case PREC_FP32: return hlld ? init_hancock_pol<PolF32, true>() : init_hancock_pol<PolF32, false>();
+    case PREC_MIXED: return hlld ? init_hancock_pol<PolMixed, true>() : init_hancock_pol<PolMixed, false>();
     default: return cudaErrorInvalidValue;
   }
 }
@@ -132,15 +131,9 @@ template <class Pol, bool HLLD, int TY, bool BATCHED>
 static cudaError_t launch_one(int stage, const Batch& b, const Member& m0, int parity, int run, int grid,
                               cudaStream_t s) {
   const size_t smem = Smem<Pol, TY>::total;
-  auto go = [&](auto* kernel) {
-    kernel<<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run, ((1u << 28) + run - 1) / run);
-    return cudaGetLastError();
-  };
-  if constexpr (kPartial<TY>) {
-    if (b.rows < tile_height(0))
-      return go(stage == 1 ? stage_kernel<Pol, 1, HLLD, TY, BATCHED, true> : stage_kernel<Pol, 2, HLLD, TY, BATCHED, true>);
-  }
-  return go(stage == 1 ? stage_kernel<Pol, 1, HLLD, TY, BATCHED, false> : stage_kernel<Pol, 2, HLLD, TY, BATCHED, false>);
+  const StageFn kernel = stage_fn<Pol, HLLD, TY, BATCHED>(stage, b.rows < tile_height(0));
+  kernel<<<grid, Geo<TY>::NT, smem, s>>>(m0, b, parity, run, ((1u << 28) + run - 1) / run);
+  return cudaGetLastError();
 }
 
 template <class Pol, int TY, bool BATCHES>
@@ -352,8 +345,8 @@ static cudaError_t launch_hancock(int precision, int hlld, int part, const Membe
 #define PMHD_TABLE_FN(n) PMHD_TABLE_FN2(n)
 
 const KernelTable& PMHD_TABLE_FN(PMHD_KNS)() {
-  static const KernelTable t = {PMHD_STR(PMHD_KNS),          PMHD_KNS::init,
-                                PMHD_KNS::launch_stage,      PMHD_KNS::ctas_per_sm,
+  static const KernelTable t = {PMHD_STR(PMHD_KNS),          PMHD_KNS::init_stage,
+                                PMHD_KNS::init_hancock,      PMHD_KNS::launch_stage,      PMHD_KNS::ctas_per_sm,
                                 PMHD_KNS::launch_speed,      PMHD_KNS::launch_aos_to_soa,
                                 PMHD_KNS::launch_soa_to_aos, PMHD_KNS::default_shape,
                                 PMHD_KNS::tile_rows,         PMHD_KNS::launch_hancock};

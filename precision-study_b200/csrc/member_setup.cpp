@@ -31,7 +31,7 @@ EncodeTiledFn encode_fn() {
 
 }  // namespace
 
-bool encode_member_tmaps(Member& m, size_t elem) {
+bool encode_member_tmaps(Member& m, size_t elem, int shapes) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return false;
   // Planes of (ny + 4) rows x pitch; the box is a tile with its 2-cell halo
@@ -41,7 +41,7 @@ bool encode_member_tmaps(Member& m, size_t elem) {
   const cuuint64_t strides[2] = {(cuuint64_t)m.pitch * elem, (cuuint64_t)m.plane * elem};
   const cuuint32_t estr[3] = {1, 1, 1};
   void* bufs[2] = {m.u, m.u1};
-  for (int t = 0; t < kNumTileShapes; t++) {
+  for (int t = 0; t < shapes; t++) {
     const cuuint32_t box[3] = {32 + 4, (cuuint32_t)tile_height(t) + 4, 9};
     for (int k = 0; k < 2; k++) {
       CUresult r = enc(&m.tm[t][k], elem == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,

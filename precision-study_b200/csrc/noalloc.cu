@@ -99,9 +99,14 @@ int setup_device(int dev, unsigned char** base) {
   if (!d.done) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || p == nullptr) return PMHD_ERR_CUDA;
-    for (int prec = PREC_FP64; prec <= PREC_MIXED; prec++)
-      if (kernel_table_exact().init(prec) != cudaSuccess || kernel_table_fast().init(prec) != cudaSuccess)
-        return PMHD_ERR_CUDA;
+    for (const KernelTable* kt : {&kernel_table_exact(), &kernel_table_fast()})
+      for (int prec = PREC_FP64; prec <= PREC_MIXED; prec++)
+        for (int hlld = 0; hlld < 2; hlld++)
+          for (int shape = 0; shape < kNumTileShapes; shape++) {
+            if (shape != 0 && shape < kNumBatchShapes) continue;  // no grid's default
+            const cudaError_t e = kt->init_stage(prec, hlld, shape, 0);
+            if (e != cudaSuccess && (shape == 0 || e != cudaErrorNotSupported)) return PMHD_ERR_CUDA;
+          }
     d.base = static_cast<unsigned char*>(p);
     d.done = true;
   }
@@ -155,7 +160,7 @@ extern "C" int pmhd_advance_noalloc(const pmhd_config* cfg, const void* d_in, vo
   hm.pitch = pitch;
   set_member_physics(hm, cfg->x_min, cfg->x_max, cfg->y_min, cfg->y_max, cfg->gamma, cfg->hlld_tol, cfg->cfl,
                      cfg->alpha, cfg->order == PMHD_ORDER_MUSCL ? 1 : 0, cfg->bc, f32);
-  if (!encode_member_tmaps(hm, elem)) return PMHD_ERR_CUDA;
+  if (!encode_member_tmaps(hm, elem, kNumTileShapes)) return PMHD_ERR_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Batch batch;
   batch.members = dmember;

@@ -71,6 +71,8 @@ cudaError_t Runner::tune(int steps, TuneResult* res) {
     // Split shapes win or lose by size, not by timing: they only run where they
     // are the default.
     if (ty >= kNumBatchShapes && ty != saved.ty_idx) continue;
+    err = kt->init_stage(precision, hlld, ty, single == nullptr);
+    if (err != cudaSuccess) break;
     const int occ = kt->ctas_per_sm(precision, hlld, ty, single == nullptr);
     for (int k = occ; k >= 1 && err == cudaSuccess; k--) {
       choice.ty_idx = ty;

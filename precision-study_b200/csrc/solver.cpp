@@ -16,7 +16,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <new>
 #include <sstream>
 #include <string>
@@ -32,9 +31,6 @@
 using namespace pmhd;
 
 namespace {
-
-std::mutex g_init_mu;
-bool g_init_done[64][2][3];
 
 }  // namespace
 
@@ -221,16 +217,11 @@ int pmhd_create(const pmhd_config* cfg, pmhd_solver** out) {
   s->cfg = *cfg;
   if (s->cfg.steps_per_graph == 0) s->cfg.steps_per_graph = 32;
   s->kt = cfg->exact ? &kernel_table_exact() : &kernel_table_fast();
-  {
-    std::lock_guard<std::mutex> lk(g_init_mu);
-    const int dev = cfg->device & 63, which = cfg->exact ? 1 : 0;
-    if (!g_init_done[dev][which][cfg->precision]) {
-      if (s->kt->init(cfg->precision) != cudaSuccess) {
-        delete s;
-        return PMHD_ERR_CUDA;
-      }
-      g_init_done[dev][which][cfg->precision] = true;
-    }
+  const int hlld = cfg->solver == PMHD_SOLVER_HLLD ? 1 : 0, shape = s->kt->default_shape(cfg->precision, cfg->nx, cfg->ny);
+  if (s->kt->init_stage(cfg->precision, hlld, shape, 0) != cudaSuccess ||
+      (cfg->order == PMHD_ORDER_HANCOCK && s->kt->init_hancock(cfg->precision, hlld) != cudaSuccess)) {
+    delete s;
+    return PMHD_ERR_CUDA;
   }
   s->elem = cfg->precision == PMHD_FP32 ? 4 : 8;
   s->pitch = ((cfg->nx + 4) + 15) / 16 * 16;
@@ -262,7 +253,7 @@ int pmhd_create(const pmhd_config* cfg, pmhd_solver** out) {
     m.pitch = s->pitch;
     set_member_physics(m, cfg->x_min, cfg->x_max, cfg->y_min, cfg->y_max, cfg->gamma, cfg->hlld_tol, cfg->cfl,
                        cfg->alpha, cfg->order == PMHD_ORDER_MUSCL ? 1 : 0, cfg->bc, is_fp32(s));
-    if (!encode_member_tmaps(m, s->elem)) rc = PMHD_ERR_CUDA;
+    if (!encode_member_tmaps(m, s->elem, kNumTileShapes)) rc = PMHD_ERR_CUDA;
     // Stream-ordered (the solver's stream does not wait for the legacy stream).
     if (rc == PMHD_OK && (cudaMemcpyAsync(s->dMember, &m, sizeof(m), cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
                           cudaStreamSynchronize(s->stream) != cudaSuccess))
@@ -271,10 +262,10 @@ int pmhd_create(const pmhd_config* cfg, pmhd_solver** out) {
     s->run.single = &s->hMember;
     s->run.kt = s->kt;
     s->run.precision = cfg->precision;
-    s->run.hlld = cfg->solver == PMHD_SOLVER_HLLD ? 1 : 0;
+    s->run.hlld = hlld;
     s->run.hancock = cfg->order == PMHD_ORDER_HANCOCK ? 1 : 0;
     s->run.stream = s->stream;
-    s->run.choice.ty_idx = s->kt->default_shape(cfg->precision, cfg->nx, cfg->ny);
+    s->run.choice.ty_idx = shape;
     for (int t = 0; t < kNumTileShapes; t++) {
       Batch& b = s->run.batch[t];
       b.members = s->dMember;
