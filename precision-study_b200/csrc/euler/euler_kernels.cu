@@ -7,8 +7,9 @@
 // 2D step kernels.  Indices are clamped at the walls (the reference's transmissive
 // ghost copies, riemann2d_cpu.cpp:160-182); the sweep order alternates with the
 // step count (even: x then y); the next step's max signal speeds come from the
-// epilogue, so the time step never needs a separate pass.  Small binary64 grids:
-// a CTA of 512 threads owns a 32 x 12 tile, loads the 36 x 16 region around it,
+// epilogue, so the time step never needs a separate pass.  Small binary64 grids
+// and most of the parity build's (see step2d): a CTA of 512 threads owns a 32 x TY
+// tile, loads the 36 x (TY + 4) region around it,
 // runs the first sweep on the part of it the second needs, then the second on the
 // tile, each as reconstruction + Hancock of every cell's two faces, one flux per
 // interface and the update, staged in shared memory.  Otherwise: the streaming
@@ -20,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstdlib>
 
 #include "euler/euler_api.h"
 #include "pmhd/euler.hpp"
@@ -646,23 +648,59 @@ int stream_rows(const StreamModel& m, int nx, int ny) {
   return best;
 }
 
-// Binary64 grids of at most one wave of 32 x 12 tiles (two 512-thread CTAs per
-// SM) run the shared-memory tile kernel, whose phases spread a step over more
-// threads: 200^2 7.9 us a step against 8.9 streaming, 500 x 197 10.9 against 12.5;
-// past one wave (400^2) 22 against 15.  Binary32 streams at every size (200^2: 6.0
-// against 8.0 us).
+// Which kernel steps a grid.  Performance build: binary64 grids of at most one
+// wave of 32 x 12 tiles (two 512-thread CTAs per SM) run the shared-memory tile
+// kernel, whose phases spread a step over more threads: 200^2 7.9 us a step against
+// 8.9 streaming, 500 x 197 10.9 against 12.5; past one wave (400^2) 22 against 15.
+// Binary32 streams at every size (200^2: 6.0 against 8.0 us).
+//
+// Parity build: its expressions take more registers (gamma is a binary64 constant in
+// binary32 too), so the streaming kernel spills and each warp's chain is longer,
+// and tiles win further up.  Us a step, tiles against streaming: binary32 32 x 32
+// 200^2 15 / 23, 1024^2 77 / 96, 3200^2 684 / 728, 3500^2 824 / 821, 4096^2 1118 /
+// 1096; binary64 32 x 16 HLLC 500^2 41 / 53, 850^2 100 / 104, 1500^2 270 / 281, 1900^2
+// 428 / 421, 4096^2 1909 / 1577; HLL 500^2 38 / 44, 750^2 73 / 73, 1024^2 125 / 113.
 constexpr int kTileH = 12, kThreads = 512;
+#if !PMHD_EULER_FAST
+constexpr int kWideH = 16, kTileH32 = 32;                 // larger tiles, binary64 / binary32
+constexpr int kWaves32 = 40, kWavesHllc = 22, kWavesHll = 4;  // tiles up to this many waves
+#endif
 
-cudaError_t prepare() { return allow_smem<double, kTileH, kThreads, 2>(); }
+long long tiles_of(int nx, int ny, int h) { return (long long)((nx + TW - 1) / TW) * ((ny + h - 1) / h); }
+
+// Test hook: PMHD_EULER_STREAM=1 streams at every size.
+bool always_stream() {
+  const char* e = std::getenv("PMHD_EULER_STREAM");
+  return e && e[0] == '1';
+}
+
+cudaError_t prepare() {
+  cudaError_t e = allow_smem<double, kTileH, kThreads, 2>();
+#if !PMHD_EULER_FAST
+  if (e == cudaSuccess) e = allow_smem<double, kWideH, kThreads, 2>();
+  if (e == cudaSuccess) e = allow_smem<float, kTileH32, kThreads, 2>();
+#endif
+  return e;
+}
 
 cudaError_t step2d(int fp32, int hll, const void* uin, void* uout, int nx, int ny, int pitch, long long plane,
                    double dx, double dy, double cfl, EulerCtrl* ctrl, int p, cudaStream_t s) {
-  if (fp32)
+  const long long wave = 2 * 148;
+  const bool tiles = !always_stream();
+  if (fp32) {
+#if !PMHD_EULER_FAST
+    if (tiles && tiles_of(nx, ny, kTileH32) <= kWaves32 * wave)
+      return launch_any<float, kTileH32, kThreads, 2>(hll, uin, uout, nx, ny, pitch, plane, dx, dy, cfl, ctrl, p, s);
+#endif
     return launch_stream<float, kStream32.cap>(hll, stream_rows(kStream32, nx, ny), uin, uout, nx, ny, pitch, plane,
                                                dx, dy, cfl, ctrl, p, s);
-  const long long tiles = (long long)((nx + TW - 1) / TW) * ((ny + kTileH - 1) / kTileH);
-  if (tiles <= 2 * 148)
+  }
+  if (tiles && tiles_of(nx, ny, kTileH) <= wave)
     return launch_any<double, kTileH, kThreads, 2>(hll, uin, uout, nx, ny, pitch, plane, dx, dy, cfl, ctrl, p, s);
+#if !PMHD_EULER_FAST
+  if (tiles && tiles_of(nx, ny, kWideH) <= (hll ? kWavesHll : kWavesHllc) * wave)
+    return launch_any<double, kWideH, kThreads, 2>(hll, uin, uout, nx, ny, pitch, plane, dx, dy, cfl, ctrl, p, s);
+#endif
   return launch_stream<double, kStream64.cap>(hll, stream_rows(kStream64, nx, ny), uin, uout, nx, ny, pitch, plane, dx,
                                               dy, cfl, ctrl, p, s);
 }
