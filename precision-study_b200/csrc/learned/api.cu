@@ -3,6 +3,8 @@
 // include/pmhd.h).
 #include <cuda_runtime.h>
 
+#include <bitset>
+#include <condition_variable>
 #include <cstdint>
 #include <mutex>
 
@@ -12,47 +14,87 @@
 
 namespace {
 
-// Error word of the calling thread's convolution calls: pinned host memory the
-// kernels write directly when a bounded wait expires, so a call needs no clearing
-// and no copy on the stream -- one launch and one synchronisation.  Every thread
-// has its own (calls are synchronous), freed when the thread ends.
-struct ErrorWord {
-  int* p = nullptr;
-  ~ErrorWord() {
-    if (p) cudaFreeHost(p);
+// Error words of the convolution calls: host memory the kernels write directly when
+// a bounded wait expires, so a call needs no clearing and no copy on the stream --
+// one launch and one synchronisation.  One page of ordinary memory, pinned by the
+// first call and kept until the process ends: the host may touch it whatever became
+// of the device's context, and no thread's start or end allocates or frees pinned
+// memory (which would wait for the device and break another thread's capture).
+// A call holds one word while it runs.
+class ErrorWords {
+ public:
+  // A cleared word and its device address; nullptr: no pinned memory, or the
+  // kernels' shared-memory limits could not be set (once per device and context).
+  int* take(int** on_device) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::unique_lock<std::mutex> lock(mu_);
+    if (cudaHostGetDevicePointer(on_device, page_, 0) != cudaSuccess) {  // first call, or the context was reset
+      cudaGetLastError();
+      for (bool& p : prepared_) p = false;
+      if (cudaHostRegister(page_, sizeof(page_), cudaHostRegisterPortable | cudaHostRegisterMapped) != cudaSuccess ||
+          cudaHostGetDevicePointer(on_device, page_, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+    }
+    if (!prepared_[dev]) {
+      if (pmhd::learned::conv_prepare() != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
+      prepared_[dev] = true;
+    }
+    given_back_.wait(lock, [this] { return busy_.count() < kWords; });
+    int k = 0;
+    while (busy_[k]) k++;
+    busy_[k] = true;
+    page_[k] = 0;
+    *on_device += k;
+    return page_ + k;
   }
+  void give_back(int* word) {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      busy_[word - page_] = false;
+    }
+    given_back_.notify_one();
+  }
+
+ private:
+  static constexpr int kWords = 1024;
+  alignas(4096) int page_[kWords];
+  std::bitset<kWords> busy_;
+  std::mutex mu_;
+  std::condition_variable given_back_;
+  bool prepared_[64] = {};
 };
 
-// The thread's error word, cleared; the first call on a device also sets the
-// kernels' shared-memory limits there.
-int* error_word() {
-  static std::mutex mu;
-  static bool prepared[64];
-  static thread_local ErrorWord word;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!prepared[dev]) {
-      if (pmhd::learned::conv_prepare() != cudaSuccess) return nullptr;
-      prepared[dev] = true;
-    }
-  }
-  if (!word.p && cudaHostAlloc(&word.p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
-    return nullptr;
-  *word.p = 0;
-  return word.p;
+ErrorWords& error_words() {
+  static ErrorWords* words = new ErrorWords;  // outlives the CUDA runtime's own statics
+  return *words;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-int finish(cudaError_t e, const int* err, cudaStream_t s) {
-  if (e == cudaErrorNotSupported) return PMHD_ERR_UNSUPPORTED;
-  if (e != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
+// One synchronous call: launch(error word on the device), wait, status.
+template <class Launch>
+int call(cudaStream_t s, Launch&& launch) {
+  int* on_device = nullptr;
+  int* word = error_words().take(&on_device);
+  if (!word) return PMHD_ERR_CUDA;
+  const cudaError_t e = launch(on_device);
+  int rc = PMHD_OK;
+  if (e == cudaErrorNotSupported) {
+    rc = PMHD_ERR_UNSUPPORTED;
+  } else if (e != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
     cudaGetLastError();
-    return PMHD_ERR_CUDA;
+    rc = PMHD_ERR_CUDA;
+  } else if (*static_cast<const volatile int*>(word)) {
+    rc = PMHD_ERR_TIMEOUT;
   }
-  return *static_cast<const volatile int*>(err) ? PMHD_ERR_TIMEOUT : PMHD_OK;
+  error_words().give_back(word);
+  return rc;
 }
 
 }  // namespace
@@ -67,26 +109,23 @@ int pmhd_conv3x3(int mode, const void* x, int batch, int h, int w, int c_in, con
   if (mode == PMHD_CONV_LINEAR && !bias) return PMHD_ERR_ARG;
   if (mode == PMHD_CONV_DGELU && (!z_prev || !aligned16(z_prev))) return PMHD_ERR_ARG;
   if (mode < PMHD_CONV_GELU || mode > PMHD_CONV_DGELU) return PMHD_ERR_ARG;
-  int* err = error_word();
-  if (!err) return PMHD_ERR_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const cudaError_t e = pmhd::learned::conv3x3(mode, static_cast<const __nv_bfloat16*>(x), batch, h, w, c_in,
-                                               static_cast<const __nv_bfloat16*>(weight), bias, c_out,
-                                               static_cast<const __nv_bfloat16*>(z_prev), out0, out1, err, s);
-  return finish(e, err, s);
+  return call(s, [&](int* err) {
+    return pmhd::learned::conv3x3(mode, static_cast<const __nv_bfloat16*>(x), batch, h, w, c_in,
+                                  static_cast<const __nv_bfloat16*>(weight), bias, c_out,
+                                  static_cast<const __nv_bfloat16*>(z_prev), out0, out1, err, s);
+  });
 }
 
 int pmhd_conv3x3_wgrad(const void* x, const void* dz, int batch, int h, int w, int c_in, int c_out, float* dweight,
                        float* dbias, void* stream) {
   if (batch < 1 || h < 1 || w < 1 || (long long)batch * h * w > (1LL << 31)) return PMHD_ERR_ARG;
   if (!x || !dz || !dweight || !aligned16(x) || !aligned16(dz)) return PMHD_ERR_ARG;
-  int* err = error_word();
-  if (!err) return PMHD_ERR_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const cudaError_t e = pmhd::learned::conv3x3_wgrad(static_cast<const __nv_bfloat16*>(x),
-                                                     static_cast<const __nv_bfloat16*>(dz), batch, h, w, c_in, c_out,
-                                                     dweight, dbias, err, s);
-  return finish(e, err, s);
+  return call(s, [&](int* err) {
+    return pmhd::learned::conv3x3_wgrad(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dz),
+                                        batch, h, w, c_in, c_out, dweight, dbias, err, s);
+  });
 }
 
 int pmhd_learned_loss_grad(const float* out, const float* tgt, int batch, int h, int w, float cx, float cy, void* dz,
