@@ -377,9 +377,10 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
       }
       __syncwarp();
     }
-    // The last two tiles' commits on empty[] have arrived before the CTA
-    // leaves (those phases are the newest of their barriers).
-    for (int kk = k - 2; ok && kk < k; kk++)
+    // The last two issued tiles' commits on empty[] have arrived before the CTA
+    // leaves, also after a failed wait: no MMA runs into released tensor memory
+    // (those phases are the newest of their barriers).
+    for (int kk = k - 2; kk < k; kk++)
       if (kk >= 0 && !warp_wait(empty + (kk & 1), (uint32_t)(kk >> 1) & 1u)) ok = false;
   } else {
     // Epilogue warps: tile k from accumulator buffer k % 2; warp q + 4 r owns
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) conv3x3_pipe_kernel(const __n
 // blocks useful).  48 MMAs of N = 64 a tile of 8 x 64 pixels.  Six producer warps
 // fill three stages; four warps sum dz for the bias gradient from the staged
 // tiles (when asked to) and add the CTA's accumulators to dw at the end.
-// 32 -> 32 over 8 x 512^2 reads 268 MB (42 us at the copy rate): about 70 us
+// 32 -> 32 over 8 x 512^2 reads 268 MB (42 us at the copy rate): 78 us
 // against 1,110 for transposing 8 x 8 blocks of nine gathered copies into K-major
 // tiles, 64 pixels at a time without overlap; 90 without swizzle (16-byte
 // planes fetch every 32-byte sector twice).
