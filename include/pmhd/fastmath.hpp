@@ -37,16 +37,23 @@ inline float fast_rsqrt(float x) { return 1.0f / std::sqrt(x); }
 inline float fast_sqrt(float x) { return std::sqrt(x); }
 #endif
 // Binary64 forms: the hardware's approximate seed (rcp / rsqrt.approx.ftz.f64,
-// about 20 bits) and one third-order step of Householder's iteration, which
-// leaves 2^-60 before the last rounding (IEEE division and square root take a
-// data-dependent slow path as well and about three times the instructions;
-// the binary64 stage kernel is bound by instruction issue and dependent
-// binary64 latency, not by a pipe).  With e = 1 - x r:  r + r (e + e^2);
-// with h = x y, e = 1 - h y:  y + y t and h + h t, t = e/2 + 3 e^2/8, the root
-// followed by one Newton correction by its residual.  fast_sqrt returns 0 and
-// +inf unchanged and NaN for negative arguments; fast_rcp and fast_rsqrt take
-// finite non-zero (positive) arguments of normal size, as their callers'
-// floors and degeneracy guards ensure.
+// about 20 bits) and one third-order step of Householder's iteration (IEEE
+// division and square root take a data-dependent slow path as well and about three
+// times the instructions; the binary64 stage kernel is bound by instruction issue
+// and dependent binary64 latency, not by a pipe).  With e = 1 - x r:  r + r (e +
+// e^2); with h = x y, e = 1 - h y:  y + y t and h + h t, t = e/2 + 3 e^2/8, the root
+// followed by one Newton correction by its residual.
+//   Errors: the step leaves the cube of the seed's error, 2^-57 or less, before the
+// last rounding: fast_rcp and the roots are within 0.6 ulp.  fast_rsqrt also carries
+// half the rounding of h (2^-54): within 1.1 ulp.
+//   Arguments: of either sign for fast_rcp, positive for the others, with argument
+// and result of normal size (2^-1022 < |x| < 2^1022; the roots keep their bound from
+// 2^-960 on, where the residual is representable).  fast_sqrt also returns 0 and +inf
+// unchanged and NaN for negative arguments.  A subnormal argument gives NaN: its
+// seed is infinite.  The callers' floors (1e-12) and degeneracy guards keep every
+// argument far inside; the Euler forms, which have no floors, meet subnormal values
+// only in states of that size, since a difference of normal values is zero or at
+// least 2^-106 of them.
 #if defined(__CUDA_ARCH__)
 __device__ __forceinline__ double fast_rcp(double x) {
   double r;
