@@ -101,6 +101,7 @@ static int occupancy() {
   std::lock_guard<std::mutex> lk(mu);
   if (per_sm < 0) {
     int nb = 0;
+    set_smem_attr<Pol, HLLD, TY, BATCHED>();  // without it the answer is 0
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stage_kernel<Pol, 1, HLLD, TY, BATCHED, false>, Geo<TY>::NT,
                                                   Smem<Pol, TY>::total);
     per_sm = nb > 0 ? nb : 1;
@@ -296,6 +297,22 @@ static cudaError_t launch_soa_to_aos(int precision, const void* u, long long pla
   return cudaGetLastError();
 }
 
+// Resident CTAs per SM of the persistent Hancock kernel.
+template <class Pol, bool HLLD>
+static int hancock_occupancy() {
+  static int per_sm = -1;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if (per_sm < 0) {
+    int nb = 0;
+    init_hancock_pol<Pol, HLLD>();  // without it the answer is 0
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, hancock_persistent_kernel<Pol, HLLD>, 256,
+                                                  sizeof(HancockTileOf<Pol>));
+    per_sm = nb > 0 ? nb : 1;
+  }
+  return per_sm;
+}
+
 template <class Pol>
 static cudaError_t hancock_pol(int hlld, int part, const Member& m, int parity, cudaStream_t s) {
   if (part == 0) {
@@ -307,13 +324,7 @@ static cudaError_t hancock_pol(int hlld, int part, const Member& m, int parity, 
   const size_t smem = sizeof(HancockTileOf<Pol>);
   if constexpr (HancockPersistent<Pol>::on) {
     // Persistent: the SMs x the resident CTAs, at most one per tile.
-    static int per_sm = -1;
-    if (per_sm < 0) {
-      int nb = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, hancock_persistent_kernel<Pol, true>, 256, smem);
-      per_sm = nb > 0 ? nb : 1;
-    }
-    int grid = sm_count() * per_sm;
+    int grid = sm_count() * (hlld ? hancock_occupancy<Pol, true>() : hancock_occupancy<Pol, false>());
     if (grid > ntiles) grid = ntiles;
     if (hlld)
       hancock_persistent_kernel<Pol, true><<<grid, 256, smem, s>>>(m, parity);

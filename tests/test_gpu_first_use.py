@@ -54,3 +54,33 @@ def test_each_way_in_works_as_the_first_of_a_process(pmhd_lib, way):
     r = subprocess.run([sys.executable, "-c", CODE % (pkg, WAYS[way], WAYS[way])], capture_output=True, text=True,
                        timeout=120)
     assert "FIRST_USE_OK" in r.stdout, r.stdout + r.stderr
+
+
+TIMED = """
+import sys
+sys.path.insert(0, %r)
+import pmhd
+best = 1e9
+for solver in %r:
+    with pmhd.Solver(nx=1024, ny=512, precision=%r, order="hancock", solver=solver) as s:
+        s.init_problem(pmhd.PROBLEM_ORSZAG_TANG)
+        s.advance(max_steps=8)
+        best = min(s.advance(max_steps=32).device_ms for _ in range(5))
+print("MS", best)
+"""
+
+
+@pytest.mark.parametrize("precision", ["fp32", "mixed"])
+def test_the_first_handle_does_not_set_the_next_ones_occupancy(pmhd_lib, precision):
+    """An HLLD handle after an HLL one runs as many CTAs per SM as one that is the first
+    of its process (half as many took 1.5 times as long)."""
+    import os
+
+    pkg = os.path.dirname(os.path.dirname(os.path.abspath(pmhd_lib.__file__)))
+    ms = {}
+    for solvers in (["hlld"], ["hll", "hlld"]):
+        r = subprocess.run([sys.executable, "-c", TIMED % (pkg, solvers, precision)], capture_output=True, text=True,
+                           timeout=120)
+        assert "MS " in r.stdout, r.stdout + r.stderr
+        ms[len(solvers)] = float(r.stdout.split("MS ")[1])
+    assert ms[2] < 1.2 * ms[1], ms
