@@ -224,12 +224,13 @@ static int default_shape(int precision, int nx, int ny) {
 // Cell rows per tile of a list of grids: the fewest with which the persistent
 // CTAs, one per SM, take no more rounds than with full 32 x 19 tiles -- a tile's
 // time falls with its rows, and the SMs a short last round leaves idle take part --
-// but 18, which full tiles beat: the 19 flux warps leave a scheduler its five, and a
-// runtime height costs 1 - 2 % (binary32 / mixed, us a step of 18-row against full
-// tiles: 288^2 21.0 / 23.6 against 20.7 / 23.4, 576^2 59.9 / 68.3 against 59.0 / 67.5,
-// 768^2 98.9 / 116.8 against 97.9 / 114.9; with 16 rows 384^2 takes 33.3 / 37.7 against
-// 33.6 / 38.4, with 17 rows 480^2 46.2 / 52.4 against 46.2 / 52.9).  Mixed, us a step,
-// of few rows against full tiles: 64^2 14.6 / 22.4, 128^2 16.1 / 22.4, 320^2 32.0 / 38.2.
+// but not 17 or 18: with rows + 1 flux warps a scheduler still has its five, and a
+// runtime height and more halo rows cost more than the other phases save (full tiles'
+// time over that of fewer rows, ten sizes each, binary32 / mixed / binary64: 17 rows
+// 0.96 - 1.01 / 0.97 - 1.03 / 0.96 - 1.02, 18 rows 0.96 - 1.00 / 0.96 - 1.01 / 0.96 - 1.00;
+// 16 rows 0.98 - 1.01 / 0.99 - 1.03 / 0.98 - 1.03, kept for their mean of 1.01; 15 rows,
+// four warps a scheduler, 1.05 - 1.12 in all).  Mixed, us a step, of few rows against
+// full tiles: 64^2 14.6 / 22.4, 128^2 16.1 / 22.4, 320^2 32.0 / 38.2.
 // The parity build's bits do not depend on the rows.  The performance build's can,
 // through tiny slopes: the tiles at the domain's edge reconstruct by minmod(), whose
 // product underflows where minmod_fast() has a value, and the rows move those tiles.
@@ -242,7 +243,7 @@ static int tile_rows(int idx, const int (*sizes)[2], int n) {
     return t;
   };
   const long long sms = sm_count(), budget = (tiles(height) + sms - 1) / sms * sms;
-  for (int rows = 2; rows < height - 1; rows++)
+  for (int rows = 2; rows < height - 2; rows++)
     if (tiles(rows) <= budget) return rows;
   return height;
 }
