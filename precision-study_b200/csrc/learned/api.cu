@@ -3,7 +3,6 @@
 // include/pmhd.h).
 #include <cuda_runtime.h>
 
-#include <bitset>
 #include <condition_variable>
 #include <cstdint>
 #include <mutex>
@@ -29,45 +28,52 @@ class ErrorWords {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::unique_lock<std::mutex> lock(mu_);
-    if (cudaHostGetDevicePointer(on_device, page_, 0) != cudaSuccess) {  // first call, or the context was reset
-      cudaGetLastError();
-      for (bool& p : prepared_) p = false;
-      if (cudaHostRegister(page_, sizeof(page_), cudaHostRegisterPortable | cudaHostRegisterMapped) != cudaSuccess ||
-          cudaHostGetDevicePointer(on_device, page_, 0) != cudaSuccess) {
+    // A reset context has lost the kernels' limits, so launches fail there until
+    // conv_prepare() runs again, and then the page is looked up (and pinned) again too.
+    if (prepared_[dev] == 0 || prepared_[dev] != pmhd::learned::conv_prepared()) {
+      int** p = &device_page_[dev];
+      cudaError_t e = cudaHostGetDevicePointer(p, page_, 0);
+      if (e != cudaSuccess) {
         cudaGetLastError();
+        e = cudaHostRegister(page_, sizeof(page_), cudaHostRegisterPortable | cudaHostRegisterMapped);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(p, page_, 0);
+      }
+      if (e == cudaSuccess) e = pmhd::learned::conv_prepare();
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        prepared_[dev] = 0;
         return nullptr;
       }
+      prepared_[dev] = pmhd::learned::conv_prepared();
     }
-    if (!prepared_[dev]) {
-      if (pmhd::learned::conv_prepare() != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-      }
-      prepared_[dev] = true;
-    }
-    given_back_.wait(lock, [this] { return busy_.count() < kWords; });
+    given_back_.wait(lock, [this] { return used_ < kWords; });
     int k = 0;
     while (busy_[k]) k++;
     busy_[k] = true;
+    used_++;
     page_[k] = 0;
-    *on_device += k;
+    *on_device = device_page_[dev] + k;
     return page_ + k;
   }
   void give_back(int* word) {
+    bool was_full;
     {
       std::lock_guard<std::mutex> lock(mu_);
       busy_[word - page_] = false;
+      was_full = used_-- == kWords;
     }
-    given_back_.notify_one();
+    if (was_full) given_back_.notify_all();
   }
 
  private:
   static constexpr int kWords = 1024;
   alignas(4096) int page_[kWords];
-  std::bitset<kWords> busy_;
+  bool busy_[kWords] = {};
+  int used_ = 0;
   std::mutex mu_;
   std::condition_variable given_back_;
-  bool prepared_[64] = {};
+  int* device_page_[64] = {};
+  unsigned prepared_[64] = {};  // conv_prepared() when the device was last looked at, 0: never
 };
 
 ErrorWords& error_words() {

@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdlib>
 
 #include "learned/conv.h"
@@ -698,7 +699,14 @@ cudaError_t launch_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dz, int ba
 
 }  // namespace
 
+namespace {
+std::atomic<unsigned> g_prepared{0};
+}
+
+unsigned conv_prepared() { return g_prepared.load(); }
+
 cudaError_t conv_prepare() {
+  g_prepared++;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);

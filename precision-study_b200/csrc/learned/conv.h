@@ -14,6 +14,8 @@ enum : int { PMHD_LEARNED_ERR_TIMEOUT = 1 };
 // Sets the kernels' shared-memory limits on the current device; call once
 // per device before the first launch (and before any stream capture).
 cudaError_t conv_prepare();
+// How often conv_prepare() has run in this process, on any device.
+unsigned conv_prepared();
 
 // One 3x3 periodic convolution over NHWC bf16 images (see conv.cu).
 //   CONV_GELU:   out0 = z = conv(x) + bias (bf16), out1 = gelu(z) (bf16)
