@@ -121,7 +121,10 @@ typedef struct {
   unsigned long long kernel_launches; /* kernels that did work, total        */
   double device_ms;                 /* GPU time of the last pmhd_advance, from
                                        CUDA events on the handle's stream     */
-  int tile_height;                  /* cell rows per stage-kernel tile     */
+  int tile_height;                  /* cell rows per stage-kernel tile; of an
+                                       ensemble and its members the height of
+                                       their tile shape (19, 8), whose tiles
+                                       cover fewer rows in short work lists     */
   int ctas;                         /* persistent CTAs per stage launch        */
   unsigned long long zone_cycles;   /* cells x steps of the last advance
                                        (summed over ensemble members)         */
@@ -218,8 +221,9 @@ int pmhd_get_config(const pmhd_solver* s, pmhd_config* cfg);
  * configuration supplies
  * precision, exact, order, solver, cfl, alpha, hlld_tol, device,
  * steps_per_graph and autotune (its nx, ny, domain, gamma and bc are
- * ignored).  Each member gives the same results as a single pmhd_solver run
- * of it. */
+ * ignored).  Each member gives the results of a single pmhd_solver run of it:
+ * the same bits when exact is 1, else up to rounding (the kernels of a batch are
+ * compiled apart from a single grid's, and small binary64 grids run other tiles). */
 typedef struct {
   int nx, ny;
   double x_min, x_max, y_min, y_max;

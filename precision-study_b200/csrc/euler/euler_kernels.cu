@@ -315,8 +315,8 @@ __global__ void __launch_bounds__(NT, MINB) step_kernel(const T* __restrict__ ui
 // in binary64, 0.57 in binary32).  Registers: 128 / 64 a thread, 16 / 32 warps per
 // SM; one-warp CTAs keep the tile position in uniform registers (four warps a CTA
 // with a position per warp: 124 bytes of spills, 10 % slower).  At 4096^2 fp64
-// 28.3 and fp32 57.8 G zone-cycles/s, against 13.2 / 26.4 with 32 x 16 / 32 x 32
-// shared-memory tiles; at 1024^2 48 / 25 us a step against 89 / 49.
+// 28.4 and fp32 56.0 G zone-cycles/s, against 12.5 / 26.0 with 32 x 16 / 32 x 32
+// shared-memory tiles; at 1024^2 48 / 25 us a step against 99 / 50.
 constexpr int kStripW = 28;
 
 template <class T>

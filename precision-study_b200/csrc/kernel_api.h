@@ -3,10 +3,10 @@
 // The kernels are compiled twice from the same source: once with IEEE
 // arithmetic and floating-point contraction disabled (-fmad=false, table
 // "exact", the bit-parity mode against the reference CPU build) and once for
-// speed (table "fast": FMA contraction, and binary32 division and square
-// root with the hardware's approximate instructions, at most 2 ulp; binary64
-// arithmetic stays IEEE apart from contraction).  solver.cpp, ensemble.cpp
-// and noalloc.cu pick a table per run.
+// speed (table "fast": FMA contraction, binary32 division and square root with
+// the hardware's approximate instructions, at most 2 ulp, and binary64
+// reciprocals and roots by pmhd/fastmath.hpp, about 1 ulp).  solver.cpp,
+// ensemble.cpp and noalloc.cu pick a table per run.
 //
 // A stage launch works on a *batch*: one or more independent grids
 // ("members", each with its own size, gamma, boundaries, time step and
@@ -38,8 +38,9 @@ constexpr int kTileShapes[kNumTileShapes] = {PMHD_TY0, 8, 8 + kSplit, 4 + kSplit
 constexpr int tile_height(int idx) { return kTileShapes[idx] & (kSplit - 1); }
 // Tiles of `rows` cell rows an nx x ny grid has.
 inline long long num_tiles(int nx, int ny, int rows) { return (long long)((nx + 31) / 32) * ((ny + rows - 1) / rows); }
-// A batched stage launch hands its CTAs runs of consecutive tiles, at most
-// this many (a power of two; see batch_run in kernels.cu).
+// A batched stage launch hands its CTAs runs of consecutive tiles, at most this many
+// (of any length for short lists, of a power of two for others: batch_run in
+// kernels.cu).
 constexpr int kBatchRunMax = 16;
 
 // One grid of a batch; lives in device memory (64-byte aligned for the TMA

@@ -540,8 +540,9 @@ __global__ void __launch_bounds__(Geo<TY>::NT, Tune<Pol, TY>::minb)
   // batch: runs of `run` consecutive tiles, run blockIdx.x, then
   // every gridDim.x-th run -- consecutive tiles of a CTA then mostly share
   // a member, so its descriptor, control slot and step values are re-read
-  // once per member run instead of once per tile, while members that stop
-  // early still leave their tiles spread over all CTAs.
+  // once per member run instead of once per tile.  The tiles of long lists stay
+  // spread over all CTAs when members stop early; those of a short list, one run a
+  // CTA, do not: the last active members' tiles sit in a few CTAs.
   // (t + 1) / run through the host's inv_run = 2^28 / run rounded up: exact for a
   // power of two, and below 2^24 tiles for the other lengths, which only lists of
   // at most 16 tiles a CTA get.  (A division here cost 1 % on long lists.)
